@@ -50,6 +50,9 @@ bool misaligned(const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 1
 }  // namespace
 
 namespace b200 {
+// gives up the scratch that the gauge force keeps between calls (gauge.cu)
+void gauge_scratch_trim();
+
 // Error reporting for the library's other translation units.
 void set_last_error(int code, const char* fmt, ...) {
   (void)code;
@@ -746,6 +749,7 @@ int b200_dwf_destroy(b200_dwf_t* op) {
   cudaFree(op->fcg_part);
   cudaFree(op->fcg_sc);
   if (op->gst) cudaStreamDestroy(op->gst);
+  gauge_scratch_trim();
   delete op;
   return 0;
 }

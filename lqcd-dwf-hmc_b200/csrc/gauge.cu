@@ -14,10 +14,13 @@
 //
 // One thread per link (site, mu) for the force and the update, one per site
 // for the action; every staple and rectangle is formed from the links it
-// touches (no shifted copies of the field are made).
+// touches (no shifted copies of the field are made).  The force reads the
+// links from a planar copy, own links go through shared memory (su3_lex.cuh).
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
+#include <mutex>
 #include <vector>
 
 #include "../../include/b200dwf.h"
@@ -36,66 +39,105 @@ struct GaugeGeom {
   __device__ size_t sh(size_t site, int mu, int d) const { return g.shift(site, mu, d); }
 };
 
+__device__ __forceinline__ void scale3(M3& a, double s) {
+#pragma unroll
+  for (int k = 0; k < 9; ++k) a.m[k] = s * a.m[k];
+}
+
 // Sum over nu != mu of the staples of U_mu(x) in the rectangle action:
 // c_plaq (upper + lower plaquette staples) + c_rect (the six 2x1 rectangles
 // through U_mu(x)), each a product S with U_mu(x) S^+ a closed loop at x.
-__device__ M3 rect_staples(const double* u, const GaugeGeom& G, size_t x, int mu, double cp, double cr) {
-  // links are re-read from global memory (L1/L2 hits) instead of being kept
-  // live, which keeps the register footprint of the 3x3 products small
+// The eight products of a plane share their factors: with the 2x1 ends
+//   A(y; a, b) = U_a(y) U_b(y+a) U_a(y+b)^+   (upper staple of U_b(y) along a)
+//   B(y; a, b) = U_a(y-a)^+ U_b(y-a) U_a(y-a+b)   (lower staple)
+// the sum is
+//   U_nu(x) { [cp V + cr A(x+nu; nu,mu)] U_nu(x+mu)^+ + cr V A(x+mu; mu,nu)^+ } + cr B(x; mu,nu) V U_nu(x+mu)^+
+// with V = U_mu(x+nu), and the mirror image below x: 22 products of 3x3
+// matrices a plane instead of 28.
+template <class F>
+__device__ __forceinline__ M3 rect_staples(const F& U, const LexHop& h, int x, int mu, double cp, double cr) {
   M3 f = zero3();
-  const size_t xpm = G.sh(x, mu, 1);
-  const size_t xmm = G.sh(x, mu, -1);
-  for (int nu = 0; nu < 4; ++nu) {
-    if (nu == mu) continue;
-    const size_t xpn = G.sh(x, nu, 1), xmn = G.sh(x, nu, -1);
-    const size_t xpmmn = G.sh(xpm, nu, -1);                    // x+mu-nu
-    // upper: U_nu(x) U_mu(x+nu) U_nu(x+mu)^+ ; lower: U_nu(x-nu)^+ U_mu(x-nu) U_nu(x-nu+mu)
-    add_to(f, mul_nd(mul_nn(G.U(u, x, nu), G.U(u, xpn, mu)), G.U(u, xpm, nu)), cp);
-    add_to(f, mul_nn(mul_dn(G.U(u, xmn, nu), G.U(u, xmn, mu)), G.U(u, xpmmn, nu)), cp);
-    if (cr == 0.0) continue;
-    const size_t xpmpn = G.sh(xpm, nu, 1);                     // x+mu+nu
-    const size_t xp2m = G.sh(xpm, mu, 1);                      // x+2mu
-    const size_t xp2n = G.sh(xpn, nu, 1);                      // x+2nu
-    const size_t xm2n = G.sh(xmn, nu, -1);                     // x-2nu
-    const size_t xmmpn = G.sh(xmm, nu, 1);                     // x-mu+nu
-    const size_t xmmmn = G.sh(xmm, nu, -1);                    // x-mu-nu
-    const size_t xp2mmn = G.sh(xp2m, nu, -1);                  // x+2mu-nu
-    const size_t xm2npm = G.sh(xm2n, mu, 1);                   // x-2nu+mu
-    // R1 = U_nu(x) U_mu(x+nu) U_mu(x+mu+nu) U_nu(x+2mu)^+ U_mu(x+mu)^+
-    add_to(f, mul_nd(mul_nd(mul_nn(mul_nn(G.U(u, x, nu), G.U(u, xpn, mu)), G.U(u, xpmpn, mu)),
-                            G.U(u, xp2m, nu)), G.U(u, xpm, mu)), cr);
-    // R2 = U_nu(x) U_nu(x+nu) U_mu(x+2nu) U_nu(x+mu+nu)^+ U_nu(x+mu)^+
-    add_to(f, mul_nd(mul_nd(mul_nn(mul_nn(G.U(u, x, nu), G.U(u, xpn, nu)), G.U(u, xp2n, mu)),
-                            G.U(u, xpmpn, nu)), G.U(u, xpm, nu)), cr);
-    // R3 = U_mu(x-mu)^+ U_nu(x-mu) U_mu(x-mu+nu) U_mu(x+nu) U_nu(x+mu)^+
-    add_to(f, mul_nd(mul_nn(mul_nn(mul_dn(G.U(u, xmm, mu), G.U(u, xmm, nu)), G.U(u, xmmpn, mu)),
-                            G.U(u, xpn, mu)), G.U(u, xpm, nu)), cr);
-    // R4 = U_nu(x-nu)^+ U_mu(x-nu) U_mu(x-nu+mu) U_nu(x-nu+2mu) U_mu(x+mu)^+
-    add_to(f, mul_nd(mul_nn(mul_nn(mul_dn(G.U(u, xmn, nu), G.U(u, xmn, mu)), G.U(u, xpmmn, mu)),
-                            G.U(u, xp2mmn, nu)), G.U(u, xpm, mu)), cr);
-    // R5 = U_nu(x-nu)^+ U_nu(x-2nu)^+ U_mu(x-2nu) U_nu(x-2nu+mu) U_nu(x-nu+mu)
-    add_to(f, mul_nn(mul_nn(mul_nn(mul_dd(G.U(u, xmn, nu), G.U(u, xm2n, nu)), G.U(u, xm2n, mu)),
-                            G.U(u, xm2npm, nu)), G.U(u, xpmmn, nu)), cr);
-    // R6 = U_mu(x-mu)^+ U_nu(x-mu-nu)^+ U_mu(x-mu-nu) U_mu(x-nu) U_nu(x-nu+mu)
-    add_to(f, mul_nn(mul_nn(mul_nn(mul_dd(G.U(u, xmm, mu), G.U(u, xmmmn, nu)), G.U(u, xmmmn, mu)),
-                            G.U(u, xmn, mu)), G.U(u, xpmmn, nu)), cr);
+  const int um = h.up(mu), dm = h.dn(mu), um2 = h.up2(mu);
+#pragma unroll 1
+  for (int k = 1; k < 4; ++k) {
+    const int nu = (mu + k) & 3;
+    const int un = h.up(nu), dn = h.dn(nu);
+    {
+      const M3 v = U.load(x + un, mu);
+      const M3 t = mul_nd(v, U.load(x + um, nu));                       // V U_nu(x+mu)^+
+      if (cr != 0.0) {
+        const M3 a1 = mul_nd(mul_nn(U.load(x + un, nu), U.load(x + h.up2(nu), mu)), U.load(x + um + un, nu));
+        M3 y = mul_nd(a1, U.load(x + um, nu));
+        const M3 a2 = mul_nd(mul_nn(U.load(x + um, mu), U.load(x + um2, nu)), U.load(x + um + un, mu));
+        mul3<false, true, true>(y, v, a2);
+        scale3(y, cr);
+        add_to(y, t, cp);
+        mul3<false, false, true>(f, U.load(x, nu), y);
+        M3 b = mul_nn(mul_dn(U.load(x + dm, mu), U.load(x + dm, nu)), U.load(x + dm + un, mu));
+        scale3(b, cr);
+        mul3<false, false, true>(f, b, t);
+      } else {
+        add_to(f, mul_nn(U.load(x, nu), t), cp);
+      }
+    }
+    {
+      const M3 v = U.load(x + dn, mu);
+      const M3 t = mul_nn(v, U.load(x + dn + um, nu));                  // V U_nu(x-nu+mu)
+      if (cr != 0.0) {
+        const int dn2 = h.dn2(nu);
+        const M3 b1 = mul_nn(mul_dn(U.load(x + dn2, nu), U.load(x + dn2, mu)), U.load(x + dn2 + um, nu));
+        M3 y = mul_nn(b1, U.load(x + dn + um, nu));
+        const M3 a2 = mul_nd(mul_nn(U.load(x + dn + um, mu), U.load(x + dn + um2, nu)), U.load(x + um, mu));
+        mul3<false, false, true>(y, v, a2);
+        scale3(y, cr);
+        add_to(y, t, cp);
+        mul3<true, false, true>(f, U.load(x + dn, nu), y);
+        M3 z = mul_nn(mul_dd(U.load(x + dm, mu), U.load(x + dm + dn, nu)), U.load(x + dm + dn, mu));
+        scale3(z, cr);
+        mul3<false, false, true>(f, z, t);
+      } else {
+        add_to(f, mul_dn(U.load(x + dn, nu), t), cp);
+      }
+    }
   }
   return f;
 }
 
-__global__ void gauge_force_kernel(const double* u, double* force, LexGeom g, double beta, double cp,
-                                   double cr) {
-  const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (idx >= 4 * g.vol) return;
-  const int mu = (int)(idx / g.vol);
-  const size_t x = idx - (size_t)mu * g.vol;
-  GaugeGeom G{g};
-  const M3 f = rect_staples(u, G, x, mu, cp, cr);
-  M3 w = mul_nd(G.U(u, x, mu), f);
-  at3(w);
+// One thread per link, a block on 128 consecutive sites of one direction
+// (blockIdx.y; four directions of 32 sites in one block, as in the stout
+// kernels, ran 1.15x slower: their 66 loads crowd each other out of L1).  Bound by
+// the latency of those loads at 8 warps an SM and by the FP64 pipe (66
+// products of 3x3 matrices a link): the five or six matrices in flight need
+// the registers of 2 resident blocks (at 3 they spill, 1.3x slower).  The
+// whole molecular-dynamics step at 16^3x32 (this kernel, momentum and link
+// update): 1096 us from lexical loads, 543 us from the planar copy.
+template <class F>
+__global__ void __launch_bounds__(128, 2) gauge_force_kernel(F u, double* force, LexGeom g, double beta, double cp,
+                                                             double cr) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int mu = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int vol = (int)g.vol;
+  const int x = blockIdx.x * 128 + threadIdx.x;
   M3 out = zero3();
-  add_to(out, w, -beta / 3.0);
-  store3(force, idx, out);
+  if (x < vol) {
+    const LexHop h(g, x);
+    const M3 f = rect_staples(u, h, x, mu, cp, cr);
+    M3 w = mul_nd(u.load(x, mu), f);
+    at3(w);
+    add_to(out, w, -beta / 3.0);
+  }
+  const size_t base = (size_t)vol * mu;
+  store3_warp(force, base + blockIdx.x * 128 + warp * 32, base + vol, buf[warp], lane, out);
+}
+
+// lexical Field_G -> planar copy
+__global__ void __launch_bounds__(128) links_to_planar_kernel(PlanarField o, const double* u) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int x = blockIdx.x * 32 + lane;
+  const size_t base = (size_t)o.vol * mu;
+  const M3 a = load3_warp(u, base + blockIdx.x * 32, base + o.vol, buf[mu], lane);
+  if (x < (int)o.vol) o.store(x, mu, a);
 }
 
 __device__ __forceinline__ double retr_nd(const M3& a, const M3& b) {   // Re tr(a b^+)
@@ -164,31 +206,72 @@ __device__ void reunit3(M3& m) {
 }
 
 // u <- reunit( (u + a iP (u + a/2 iP ( ... (u + a/n iP u) ...))) ), n = nprec
-__global__ void link_update_kernel(double* u, const double* ip, size_t nlink, double alpha, int nprec) {
-  const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (idx >= nlink) return;
-  const M3 u0 = load3(u, idx);
-  const M3 iv = load3(ip, idx);
+__global__ void __launch_bounds__(128) link_update_kernel(double* u, const double* ip, size_t nlink, double alpha,
+                                                          int nprec) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t first = blockIdx.x * (size_t)128 + warp * 32;
+  const M3 u0 = load3_warp(u, first, nlink, buf[warp], lane);
+  const M3 iv = load3_warp(ip, first, nlink, buf[warp], lane);
   M3 t = u0;
-  for (int k = 0; k < nprec; ++k) {
-    const double f = alpha / (double)(nprec - k);
-    M3 p = mul_nn(iv, t);
-    t = u0;
-    add_to(t, p, f);
+  if (first + lane < nlink) {
+    for (int k = 0; k < nprec; ++k) {
+      const double f = alpha / (double)(nprec - k);
+      const M3 p = mul_nn(iv, t);
+      t = u0;
+      add_to(t, p, f);
+    }
+    reunit3(t);
   }
-  reunit3(t);
-  store3(u, idx, t);
+  store3_warp(u, first, nlink, buf[warp], lane, t);
 }
 
-__global__ void axpy_links_kernel(double* y, const double* x, size_t n, double a) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = fma(a, x[i], y[i]);
+// y = a x + b y over link fields of n elements (b = 0: y = a x, y not read).
+// HBM-bound: four independent 16-byte loads of each operand a thread keep
+// enough bytes in flight (8-byte loads, one at a time, did not); T is double
+// only for arrays that are not 16-byte aligned.
+constexpr int kAxpyUnroll = 4;
+__device__ __forceinline__ double axpby1(double a, double x, double b, double y) { return fma(a, x, b * y); }
+__device__ __forceinline__ double2 axpby1(double a, double2 x, double b, double2 y) {
+  return make_double2(fma(a, x.x, b * y.x), fma(a, x.y, b * y.y));
+}
+__device__ __forceinline__ double scale1(double a, double x) { return a * x; }
+__device__ __forceinline__ double2 scale1(double a, double2 x) { return make_double2(a * x.x, a * x.y); }
+
+template <typename T, bool kReadY>
+__global__ void __launch_bounds__(256) axpby_links_kernel(T* y, const T* x, size_t n, double a, double b) {
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += kAxpyUnroll * step) {
+    T xv[kAxpyUnroll], yv[kAxpyUnroll];
+#pragma unroll
+    for (int k = 0; k < kAxpyUnroll; ++k) {
+      const size_t j = i + k * step;
+      if (j < n) {
+        xv[k] = x[j];
+        if (kReadY) yv[k] = y[j];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAxpyUnroll; ++k) {
+      const size_t j = i + k * step;
+      if (j < n) y[j] = kReadY ? axpby1(a, xv[k], b, yv[k]) : scale1(a, xv[k]);
+    }
+  }
 }
 
-// y = a x + b y over link fields (b = 0: y = a x, y not read)
-__global__ void axpby_links_kernel(double* y, const double* x, size_t n, double a, double b) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = (b == 0.0) ? a * x[i] : fma(a, x[i], b * y[i]);
+template <typename T>
+cudaError_t run_axpby_links(double* y, const double* x, size_t n, double a, double b, cudaStream_t st) {
+  const size_t m = n * sizeof(double) / sizeof(T);           // n is a multiple of 18
+  const size_t want = (m + 256 * kAxpyUnroll - 1) / (256 * kAxpyUnroll);
+  const int nb = (int)(want < 148 * 8 ? want : 148 * 8);
+  if (b == 0.0) axpby_links_kernel<T, false><<<nb, 256, 0, st>>>((T*)y, (const T*)x, m, a, b);
+  else axpby_links_kernel<T, true><<<nb, 256, 0, st>>>((T*)y, (const T*)x, m, a, b);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_axpby_links(double* y, const double* x, size_t n, double a, double b, cudaStream_t st) {
+  const bool wide = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
+  return wide ? run_axpby_links<double2>(y, x, n, a, b, st) : run_axpby_links<double>(y, x, n, a, b, st);
 }
 
 // iP = i sum_a h_a lambda_a on every link (Langevin_Momentum::set_iP_SU3,
@@ -258,7 +341,50 @@ int fail_code(int code, const char* msg) {
     }                                                                                  \
   } while (0)
 
+// Scratch of the gauge force (a planar copy of the links): stream-ordered
+// allocations from a pool of this library, one per device, so that calls on
+// several streams and threads each have their own and a repeated call does
+// not wait for the allocator.  At most kPoolKeep bytes stay with the pool
+// between calls; gauge_scratch_trim (run when a plan is destroyed) gives them
+// back.
+constexpr int kMaxDevices = 64;
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+
+cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&g_pool[dev], &props) != cudaSuccess) {
+      cudaGetLastError();
+      g_pool[dev] = nullptr;
+    } else {
+      cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+  }
+  return g_pool[dev];
+}
+
 }  // namespace
+
+void gauge_scratch_trim() {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (int d = 0; d < kMaxDevices; ++d)
+    if (g_pool[d]) cudaMemPoolTrimTo(g_pool[d], 0);
+}
+
+cudaError_t launch_links_to_planar(double2* out, const double* u, size_t vol, cudaStream_t st) {
+  links_to_planar_kernel<<<(unsigned)((vol + 31) / 32), 128, 0, st>>>(PlanarField{out, (unsigned)vol}, u);
+  return cudaGetLastError();
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -269,10 +395,28 @@ int b200_gauge_force_rect(const int lattice[4], double beta, double c_plaq, doub
                           const double* u, void* stream) {
   LexGeom g;
   if (!geom_ok(lattice, &g) || !force || !u) return fail_code(B200_EINVAL, "invalid argument");
-  const size_t n = 4 * g.vol;
-  gauge_force_kernel<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(u, force, g, beta, c_plaq,
-                                                                                     c_rect);
-  G_CHECK(cudaGetLastError());
+  if (g.vol > 0x7fffffffu) return fail_code(B200_EINVAL, "lattice volume too large");
+  cudaStream_t st = (cudaStream_t)stream;
+  const dim3 grid((unsigned)((g.vol + 127) / 128), 4);
+  // The planar copy costs one pass over the links and makes the 66 link loads
+  // of a thread whole lines; without room for it the links are read where
+  // they are (same arithmetic, 16^3x32: 3.5x slower).
+  double2* planar = nullptr;
+  cudaMemPool_t pool = scratch_pool();
+  if (!pool || cudaMallocFromPoolAsync((void**)&planar, 4 * g.vol * 9 * sizeof(double2), pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    gauge_force_kernel<<<grid, 128, 0, st>>>(LexField{u, (unsigned)g.vol}, force, g, beta, c_plaq, c_rect);
+    G_CHECK(cudaGetLastError());
+    return 0;
+  }
+  cudaError_t e = launch_links_to_planar(planar, u, g.vol, st);
+  if (e == cudaSuccess) {
+    gauge_force_kernel<<<grid, 128, 0, st>>>(PlanarField{planar, (unsigned)g.vol}, force, g, beta, c_plaq, c_rect);
+    e = cudaGetLastError();
+  }
+  const cudaError_t ef = cudaFreeAsync(planar, st);
+  G_CHECK(e);
+  G_CHECK(ef);
   return 0;
 }
 
@@ -311,8 +455,7 @@ int b200_momentum_update(const int lattice[4], double eps, const double* force, 
   LexGeom g;
   if (!geom_ok(lattice, &g) || !force || !ip) return fail_code(B200_EINVAL, "invalid argument");
   const size_t n = 18 * 4 * g.vol;
-  axpy_links_kernel<<<592, 256, 0, (cudaStream_t)stream>>>(ip, force, n, eps);
-  G_CHECK(cudaGetLastError());
+  G_CHECK(launch_axpby_links(ip, force, n, eps, 1.0, (cudaStream_t)stream));
   return 0;
 }
 
@@ -339,8 +482,7 @@ int b200_momentum_energy(const int lattice[4], const double* ip, double* H, void
 int b200_links_axpby(const int lattice[4], double a, const double* x, double b, double* y, void* stream) {
   LexGeom g;
   if (!geom_ok(lattice, &g) || !x || !y) return fail_code(B200_EINVAL, "invalid argument");
-  axpby_links_kernel<<<592, 256, 0, (cudaStream_t)stream>>>(y, x, 18 * 4 * g.vol, a, b);
-  G_CHECK(cudaGetLastError());
+  G_CHECK(launch_axpby_links(y, x, 18 * 4 * g.vol, a, b, (cudaStream_t)stream));
   return 0;
 }
 

@@ -14,6 +14,9 @@
 // ri + 2*(col + 3*row) + 18*(site + Nvol*mu).
 #include <cuda_runtime.h>
 
+#include <mutex>
+#include <vector>
+
 #include "../../include/b200dwf.h"
 #include "dwf_kernels.h"
 #include "su3_lex.cuh"
@@ -22,23 +25,20 @@ namespace b200 {
 
 
 // rho * sum_{nu != mu} (upper + lower) staples of U_mu(x)
-__device__ M3 staple_sum(const double* u, const LexGeom& g, size_t site, int mu, double rho) {
+__device__ __forceinline__ M3 staple_sum(const PlanarField& u, const LexHop& h, int x, int mu, double rho) {
   M3 c = zero3();
-  const size_t xmu = g.shift(site, mu, 1);
-  for (int nu = 0; nu < 4; ++nu) {
-    if (nu == mu) continue;
-    const size_t xnu = g.shift(site, nu, 1);
-    const size_t xmnu = g.shift(site, nu, -1);
-    const size_t xmnu_mu = g.shift(xmnu, mu, 1);
+  const int um = h.up(mu);
+#pragma unroll 1
+  for (int k = 1; k < 4; ++k) {
+    const int nu = (mu + k) & 3;
+    const int un = h.up(nu), dn = h.dn(nu);
     // U_nu(x) U_mu(x+nu) U_nu(x+mu)^+
-    const M3 up = mul_nd(mul_nn(load3(u, site + g.vol * nu), load3(u, xnu + g.vol * mu)),
-                         load3(u, xmu + g.vol * nu));
+    mul3<false, true, true>(c, mul_nn(u.load(x, nu), u.load(x + un, mu)), u.load(x + um, nu));
     // U_nu(x-nu)^+ U_mu(x-nu) U_nu(x-nu+mu)
-    const M3 dn = mul_nn(mul_dn(load3(u, xmnu + g.vol * nu), load3(u, xmnu + g.vol * mu)),
-                         load3(u, xmnu_mu + g.vol * nu));
-    add_to(c, up, rho);
-    add_to(c, dn, rho);
+    mul3<false, false, true>(c, mul_dn(u.load(x + dn, nu), u.load(x + dn, mu)), u.load(x + dn + um, nu));
   }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) c.m[k] = rho * c.m[k];
   return c;
 }
 
@@ -56,15 +56,12 @@ __device__ M3 staple_sum(const double* u, const LexGeom& g, size_t site, int mu,
 // d f_j/dc1 (-c0) = (-1)^j conj(...) and d f_j/dc0 (-c0) = (-1)^(j+1) conj(...).
 // ---------------------------------------------------------------------------
 
-// sin(w)/w
-__device__ __forceinline__ double sinc_w(double w) { return (w == 0.0) ? 1.0 : sin(w) / w; }
-
-// (cos w - sin(w)/w) / w^2 = d/dw (sin(w)/w) / w.  For small w, where the
-// closed form cancels, its Taylor series
+// (cos w - sin(w)/w) / w^2 = d/dw (sin(w)/w) / w, from w, sin w and cos w.
+// For small w, where the closed form cancels, its Taylor series
 //   sum_m (-1)^(m+1) (2m+2) w^(2m) / (2m+3)!
 // is summed term by term (each term from the previous one).
-__device__ double dsinc_w(double w) {
-  if (w >= 0.5) return (cos(w) - sin(w) / w) / (w * w);
+__device__ double dsinc_w(double w, double sinw, double cosw) {
+  if (w >= 0.5) return (cosw - sinw / w) / (w * w);
   const double w2 = w * w;
   double term = -1.0 / 3.0, sum = 0.0;
   for (int m = 1; m < 12; ++m) {
@@ -80,7 +77,11 @@ struct ExpCoef {
   Cx d0[3];    // d f_j / d c0
 };
 
-__device__ __forceinline__ Cx expi(double a) { return cx(cos(a), sin(a)); }
+__device__ __forceinline__ Cx expi(double a) {
+  Cx e;
+  sincos(a, &e.i, &e.r);
+  return e;
+}
 __device__ __forceinline__ Cx imul(double s, Cx a) { return cx(-s * a.i, s * a.r); }   // i s a
 
 // kDeriv: also the derivatives (the force's B1, B2)
@@ -90,12 +91,16 @@ __device__ ExpCoef expi_coef(double c0, double c1) {
   const double a0 = fabs(c0);
   const double s3 = sqrt(c1 / 3.0);
   const double theta = acos(fmin(1.0, a0 / (2.0 * s3 * s3 * s3)));
-  const double u = s3 * cos(theta / 3.0);
-  const double w = sqrt(c1) * sin(theta / 3.0);
+  double st, ct, sw, cw;
+  sincos(theta / 3.0, &st, &ct);
+  const double u = s3 * ct;
+  const double w = sqrt(c1) * st;
   const double uu = u * u, ww = w * w;
-  const double sw = sinc_w(w), cw = cos(w);
-  const Cx p2 = expi(2.0 * u);      // e^{2iu}
-  const Cx m1 = expi(-u);           // e^{-iu}
+  sincos(w, &sw, &cw);
+  const double ds = kDeriv ? dsinc_w(w, sw, cw) : 0.0;
+  sw = (w == 0.0) ? 1.0 : sw / w;            // sin(w)/w
+  const Cx m1 = expi(-u);                    // e^{-iu}
+  const Cx p2 = conj(m1) * conj(m1);         // e^{2iu}
   const double den = 9.0 * uu - ww;
   ExpCoef r;
   // h_j / (9u^2 - w^2), paper eqs. (30)-(33)
@@ -103,7 +108,6 @@ __device__ ExpCoef expi_coef(double c0, double c1) {
   r.f[1] = (1.0 / den) * ((2.0 * u) * p2 - m1 * cx(2.0 * u * cw, -(3.0 * uu - ww) * sw));
   r.f[2] = (1.0 / den) * (p2 - m1 * cx(cw, 3.0 * u * sw));
   if (kDeriv) {
-    const double ds = dsinc_w(w);
     // the paper's r_j^(1), r_j^(2) (eqs. 58-60), written out per component
     Cx ra[3], rb[3];
     ra[0] = 2.0 * (cx(u, uu - ww) * p2) +
@@ -182,29 +186,50 @@ __device__ __forceinline__ StoutQ stout_q(const M3& C, const M3& U) {
 __device__ __forceinline__ bool stout_negligible(const StoutQ& q) { return 2.0 * q.c1 <= 1.0e-10; }
 
 struct StoutParams {
-  const double* u;     // links of this level (input of the smearing step)
-  double* u_out;       // smeared links
-  const double* sigp;  // force w.r.t. the smeared links
-  double* sig;         // force w.r.t. u (output)
-  double* itheta;      // per-link Theta (recursive -> force_each)
+  PlanarField u;          // links of this level (input of the smearing step)
+  PlanarField out;        // smeared links, planar (p null: not wanted)
+  double* out_lex;        // smeared links, lexical (null: not wanted)
+  PlanarField sig;        // force w.r.t. the smeared links in, w.r.t. u out
+  const double* sig_in;   // the force arrives here in the lexical layout (null: in sig)
+  double* sig_out;        // the finished force goes here in the lexical layout (null: to sig)
+  PlanarField itheta;     // per-link i Theta (recursive -> force_each)
   double rho;
   LexGeom g;
 };
 
-// U' = exp(iQ) U, one thread per link
-__global__ void stout_smear_kernel(StoutParams p) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 4 * p.g.vol) return;
-  const int mu = (int)(idx / p.g.vol);
-  const size_t site = idx % p.g.vol;
-  const M3 U = load3(p.u, idx);
-  const StoutQ q = stout_q(staple_sum(p.u, p.g, site, mu, p.rho), U);
-  if (stout_negligible(q)) {
-    store3(p.u_out, idx, U);
-    return;
+// The kernels below run one thread per link, a block on the four directions
+// (one a warp) of 32 consecutive sites, so that the directions find each
+// other's links in L1 and L2, and read neighbours from planar copies
+// (su3_lex.cuh).  They are bound by the FP64 pipe (12 products of 3x3
+// matrices a link for the staples, 30 in force_each; 45 % busy) and, at the 8
+// to 12 warps an SM that their registers leave, by the latency of the loads;
+// at 4 resident blocks they spill and run 1.1-1.7x slower.  Two levels and the
+// Jacobian at 24^3x48: 10.8 ms from lexical loads with 64-bit index divisions,
+// 5.7 ms from the planar copies.
+
+// U' = exp(iQ) U
+__global__ void __launch_bounds__(128, 3) stout_smear_kernel(StoutParams p) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int vol = (int)p.g.vol;
+  const int x = blockIdx.x * 32 + lane;
+  M3 o = zero3();
+  if (x < vol) {
+    const LexHop h(p.g, x);
+    const M3 U = p.u.load(x, mu);
+    const StoutQ q = stout_q(staple_sum(p.u, h, x, mu, p.rho), U);
+    if (stout_negligible(q)) {
+      o = U;
+    } else {
+      const ExpCoef k = expi_coef<false>(q.c0, q.c1);
+      o = mul_nn(qpoly(k.f, q.Q, q.Q2), U);
+    }
+    if (p.out.p) p.out.store(x, mu, o);
   }
-  const ExpCoef k = expi_coef<false>(q.c0, q.c1);
-  store3(p.u_out, idx, mul_nn(qpoly(k.f, q.Q, q.Q2), U));
+  if (p.out_lex) {
+    const size_t base = (size_t)vol * mu;
+    store3_warp(p.out_lex, base + blockIdx.x * 32, base + vol, buf[mu], lane, o);
+  }
 }
 
 // One backward step of the stout chain for link (x, mu): with M = U Sigma'
@@ -212,14 +237,22 @@ __global__ void stout_smear_kernel(StoutParams p) {
 //   iLambda = TA(i Gamma),   iTheta = iLambda U   (kept for force_each)
 //   Sigma  = Sigma' exp(iQ) + C^+ iLambda
 // (paper eqs. 69-75); the staple derivative terms follow in force_each.
-__global__ void stout_recursive_kernel(StoutParams p) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 4 * p.g.vol) return;
-  const int mu = (int)(idx / p.g.vol);
-  const size_t site = idx % p.g.vol;
-  const M3 U = load3(p.u, idx);
-  const M3 C = staple_sum(p.u, p.g, site, mu, p.rho);
-  const M3 Sp = load3(p.sigp, idx);
+// Sigma' and Sigma are the thread's own link only, so sig is updated in place.
+__global__ void __launch_bounds__(128, 2) stout_recursive_kernel(StoutParams p) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int vol = (int)p.g.vol;
+  const int x = blockIdx.x * 32 + lane;
+  M3 Sp;
+  if (p.sig_in) {
+    const size_t base = (size_t)vol * mu;
+    Sp = load3_warp(p.sig_in, base + blockIdx.x * 32, base + vol, buf[mu], lane);
+  }
+  if (x >= vol) return;
+  if (!p.sig_in) Sp = p.sig.load(x, mu);
+  const LexHop h(p.g, x);
+  const M3 U = p.u.load(x, mu);
+  const M3 C = staple_sum(p.u, h, x, mu, p.rho);
   const StoutQ q = stout_q(C, U);
   M3 e, il;
   if (stout_negligible(q)) {
@@ -231,73 +264,94 @@ __global__ void stout_recursive_kernel(StoutParams p) {
     const M3 M = mul_nn(U, Sp);
     const Cx g1 = tr_mul(M, qpoly(k.d1, q.Q, q.Q2));
     const Cx g0 = tr_mul(M, qpoly(k.d0, q.Q, q.Q2));
-    const M3 QM = mul_nn(q.Q, M);
-    const M3 MQ = mul_nn(M, q.Q);
+    M3 QM = mul_nn(q.Q, M);
+    mul3<false, false, true>(QM, M, q.Q);
 #pragma unroll
     for (int n = 0; n < 9; ++n) {
-      const Cx gam = g1 * q.Q.m[n] + g0 * q.Q2.m[n] + k.f[1] * M.m[n] + k.f[2] * (QM.m[n] + MQ.m[n]);
+      Cx gam = g1 * q.Q.m[n];
+      cmac(gam, g0, q.Q2.m[n]);
+      cmac(gam, k.f[1], M.m[n]);
+      cmac(gam, k.f[2], QM.m[n]);
       il.m[n] = imul(1.0, gam);
     }
     at3(il);
   }
-  store3(p.itheta, idx, mul_nn(il, U));
+  p.itheta.store(x, mu, mul_nn(il, U));
   M3 sig = mul_nn(Sp, e);
-  add_to(sig, mul_dn(C, il));
-  store3(p.sig, idx, sig);
+  mul3<true, false, true>(sig, C, il);
+  p.sig.store(x, mu, sig);
 }
 
-// ForceSmear_APE::force_each summed over nu != mu, times rho, added to sig
-__global__ void stout_force_each_kernel(StoutParams p) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 4 * p.g.vol) return;
-  const int mu = (int)(idx / p.g.vol);
-  const size_t x = idx % p.g.vol;
-  const size_t V = p.g.vol;
-  const double* U = p.u;
-  const double* T = p.itheta;
+// ForceSmear_APE::force_each summed over nu != mu, times rho, added to sig.
+// Six products a plane and side, two of which share their outer factor:
+//   above x:  V_nu(x+mu) [V_mu(x+nu)^+ iT_nu(x)^+ + iT_mu(x+nu)^+ V_nu(x)^+] + iT_nu(x+mu) V_mu(x+nu)^+ V_nu(x)^+
+//   below:    V_nu(y+mu)^+ [iT_mu(y)^+ V_nu(y) + V_mu(y)^+ iT_nu(y)] + iT_nu(y+mu)^+ V_mu(y)^+ V_nu(y),  y = x - nu
+__global__ void __launch_bounds__(128, 2) stout_force_each_kernel(StoutParams p) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int vol = (int)p.g.vol;
+  const int x = blockIdx.x * 32 + lane;
+  const PlanarField& U = p.u;
+  const PlanarField& T = p.itheta;
   M3 acc = zero3();
-  const size_t xmu = p.g.shift(x, mu, 1);
-  for (int nu = 0; nu < 4; ++nu) {
-    if (nu == mu) continue;
-    const size_t xnu = p.g.shift(x, nu, 1);
-    const size_t xmn = p.g.shift(x, nu, -1);          // x - nu
-    const size_t xmn_mu = p.g.shift(xmn, mu, 1);      // x - nu + mu
-    const M3 Vnu_xmu = load3(U, xmu + V * nu);
-    const M3 Vmu_xnu = load3(U, xnu + V * mu);
-    const M3 Vnu_x = load3(U, x + V * nu);
-    M3 s = zero3();
-    // V_nu(x+mu) V_mu(x+nu)^+ iT_nu(x)^+
-    add_to(s, mul_nd(mul_nd(Vnu_xmu, Vmu_xnu), load3(T, x + V * nu)));
-    // V_nu(x-nu+mu)^+ iT_mu(x-nu)^+ V_nu(x-nu)
-    const M3 Vnu_xmnmu = load3(U, xmn_mu + V * nu);
-    const M3 Vnu_xmn = load3(U, xmn + V * nu);
-    add_to(s, mul_dn(Vnu_xmnmu, mul_dn(load3(T, xmn + V * mu), Vnu_xmn)));
-    // V_nu(x-nu+mu)^+ V_mu(x-nu)^+ iT_nu(x-nu)
-    const M3 Vmu_xmn = load3(U, xmn + V * mu);
-    add_to(s, mul_dn(Vnu_xmnmu, mul_dn(Vmu_xmn, load3(T, xmn + V * nu))));
-    // iT_nu(x+mu) V_mu(x+nu)^+ V_nu(x)^+
-    add_to(s, mul_nd(mul_nd(load3(T, xmu + V * nu), Vmu_xnu), Vnu_x));
-    // iT_nu(x-nu+mu)^+ V_mu(x-nu)^+ V_nu(x-nu)
-    add_to(s, mul_nn(mul_dd(load3(T, xmn_mu + V * nu), Vmu_xmn), Vnu_xmn));
-    // V_nu(x+mu) iT_mu(x+nu)^+ V_nu(x)^+
-    add_to(s, mul_nd(mul_nd(Vnu_xmu, load3(T, xnu + V * mu)), Vnu_x));
-    add_to(acc, s, p.rho);
+  if (x < vol) {
+    const LexHop h(p.g, x);
+    const int um = h.up(mu);
+#pragma unroll 1
+    for (int k = 1; k < 4; ++k) {
+      const int nu = (mu + k) & 3;
+      const int un = h.up(nu);
+      {
+        const M3 vm = U.load(x + un, mu), vn = U.load(x, nu);
+        M3 s = mul_dd(vm, T.load(x, nu));
+        mul3<true, true, true>(s, T.load(x + un, mu), vn);
+        mul3<false, false, true>(acc, U.load(x + um, nu), s);
+        mul3<false, true, true>(acc, mul_nd(T.load(x + um, nu), vm), vn);
+      }
+      {
+        const int y = x + h.dn(nu);
+        const M3 vm = U.load(y, mu), vn = U.load(y, nu);
+        M3 s = mul_dn(T.load(y, mu), vn);
+        mul3<true, false, true>(s, vm, T.load(y, nu));
+        mul3<true, false, true>(acc, U.load(y + um, nu), s);
+        mul3<false, false, true>(acc, mul_dd(T.load(y + um, nu), vm), vn);
+      }
+    }
+    M3 out = p.sig.load(x, mu);
+    add_to(out, acc, p.rho);
+    acc = out;
+    if (!p.sig_out) p.sig.store(x, mu, acc);
   }
-  M3 out = load3(p.sig, idx);
-  add_to(out, acc);
-  store3(p.sig, idx, out);
+  if (p.sig_out) {
+    const size_t base = (size_t)vol * mu;
+    store3_warp(p.sig_out, base + blockIdx.x * 32, base + vol, buf[mu], lane, acc);
+  }
+}
+
+// planar -> lexical Field_G
+__global__ void __launch_bounds__(128) planar_to_links_kernel(double* out, PlanarField in) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const int x = blockIdx.x * 32 + lane;
+  M3 a = zero3();
+  if (x < (int)in.vol) a = in.load(x, mu);
+  const size_t base = (size_t)in.vol * mu;
+  store3_warp(out, base + blockIdx.x * 32, base + in.vol, buf[mu], lane, a);
 }
 
 // AForce_F<ACCEL>::mult_generator (src/lib_alt_Accel/Force/Fermion/aforce_F.cpp:62-75):
 // F_mu(x) <- -2 at(U_mu(x) F_mu(x))
-__global__ void mult_generator_kernel(double* f, const double* u, size_t nlink) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nlink) return;
-  M3 m = mul_nn(load3(u, idx), load3(f, idx));
+__global__ void __launch_bounds__(128) mult_generator_kernel(double* f, const double* u, size_t nlink) {
+  __shared__ double2 buf[4][kLinkBuf];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t first = blockIdx.x * (size_t)128 + warp * 32;
+  const M3 a = load3_warp(u, first, nlink, buf[warp], lane);
+  const M3 b = load3_warp(f, first, nlink, buf[warp], lane);
+  M3 m = mul_nn(a, b);
   at3(m);
 #pragma unroll
   for (int k = 0; k < 9; ++k) m.m[k] = -2.0 * m.m[k];
-  store3(f, idx, m);
+  store3_warp(f, first, nlink, buf[warp], lane, m);
 }
 
 }  // namespace b200
@@ -305,13 +359,20 @@ __global__ void mult_generator_kernel(double* f, const double* u, size_t nlink) 
 // ------------------------------------------------------------ smearing plan
 using namespace b200;
 
+// Levels 0 .. nsmear-1 are kept planar (what the next level and the Jacobian
+// read), the top level in the lexical layout (what callers read).  Another
+// level asked for by b200_smear_config gets a lexical copy then, refreshed by
+// every later set_config, so the pointer handed out stays that level's.
 struct b200_smear {
   LexGeom g;
   double rho;
   int nsmear;
-  double* levels = nullptr;   // (nsmear + 1) configs, level 0 = thin links
-  double* itheta = nullptr;
-  double* sig_tmp = nullptr;
+  double2* block = nullptr;        // one allocation: the top level, then the arrays below
+  double2* planar = nullptr;       // nsmear planar levels
+  std::vector<double*> lex;        // lexical copies per level (top: in block)
+  double2* itheta = nullptr;
+  double2* sig = nullptr;
+  std::mutex mu;                   // guards the lexical copies made on request
   bool have_config = false;
 };
 
@@ -345,13 +406,20 @@ int b200_smear_create(b200_smear_t** out, const int lattice[4], double rho, int 
   sm->g.vol = (size_t)lattice[0] * lattice[1] * lattice[2] * lattice[3];
   sm->rho = rho;
   sm->nsmear = nsmear;
-  const size_t n = nreal_cfg(sm) * sizeof(double);
-  if (cudaMalloc(&sm->levels, (nsmear + 1) * n) != cudaSuccess ||
-      cudaMalloc(&sm->itheta, n) != cudaSuccess || cudaMalloc(&sm->sig_tmp, n) != cudaSuccess) {
-    cudaFree(sm->levels); cudaFree(sm->itheta); cudaFree(sm->sig_tmp);
-    delete sm;
+  sm->lex.assign(nsmear + 1, nullptr);
+  const size_t n = nreal_cfg(sm) / 2;      // double2 of one field
+  const size_t fields = nsmear > 0 ? nsmear + 3 : 1;
+  if (sm->g.vol > 0x7fffffffu || cudaMalloc(&sm->block, fields * n * sizeof(double2)) != cudaSuccess) {
+    sm->block = nullptr;
+    b200_smear_destroy(sm);
     set_last_error(B200_ENOMEM, "smear_create: device allocation failed");
     return B200_ENOMEM;
+  }
+  sm->lex[nsmear] = reinterpret_cast<double*>(sm->block);
+  if (nsmear > 0) {
+    sm->itheta = sm->block + n;
+    sm->sig = sm->block + 2 * n;
+    sm->planar = sm->block + 3 * n;
   }
   *out = sm;
   return 0;
@@ -359,27 +427,45 @@ int b200_smear_create(b200_smear_t** out, const int lattice[4], double rho, int 
 
 int b200_smear_destroy(b200_smear_t* sm) {
   if (!sm) return 0;
-  cudaFree(sm->levels);
-  cudaFree(sm->itheta);
-  cudaFree(sm->sig_tmp);
+  for (int i = 0; i < sm->nsmear; ++i) cudaFree(sm->lex[i]);
+  cudaFree(sm->block);
+  gauge_scratch_trim();
   delete sm;
   return 0;
 }
 
+static PlanarField planar_level(const b200_smear* sm, int level) {
+  return PlanarField{sm->planar + (size_t)level * 36 * sm->g.vol, (unsigned)sm->g.vol};
+}
+
+static unsigned link_grid(const b200_smear* sm) { return (unsigned)((sm->g.vol + 31) / 32); }
+
 int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void* stream) {
   if (!sm || !u) { set_last_error(B200_EINVAL, "smear_set_config: invalid argument"); return B200_EINVAL; }
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t n = nreal_cfg(sm);
-  B200_SMEAR_CHECK(cudaMemcpyAsync(sm->levels, u, n * sizeof(double),
-                                   on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
-  const int grid = (int)((4 * sm->g.vol + 127) / 128);
+  const size_t bytes = nreal_cfg(sm) * sizeof(double);
+  std::lock_guard<std::mutex> lock(sm->mu);
+  double* top = sm->lex[sm->nsmear];
+  const double* thin = u;
+  if (sm->nsmear == 0 || !on_device) {
+    // host links pass through the top level's buffer, which the last level
+    // overwrites once the planar copy has been made
+    B200_SMEAR_CHECK(cudaMemcpyAsync(top, u, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+    thin = top;
+  }
+  if (sm->nsmear > 0) B200_SMEAR_CHECK(launch_links_to_planar(planar_level(sm, 0).p, thin, sm->g.vol, st));
   for (int i = 0; i < sm->nsmear; ++i) {
     StoutParams p{};
-    p.u = sm->levels + i * n;
-    p.u_out = sm->levels + (i + 1) * n;
+    p.u = planar_level(sm, i);
+    if (i + 1 < sm->nsmear) p.out = planar_level(sm, i + 1);
+    p.out_lex = sm->lex[i + 1];
     p.rho = sm->rho;
     p.g = sm->g;
-    stout_smear_kernel<<<grid, 128, 0, st>>>(p);
+    stout_smear_kernel<<<link_grid(sm), 128, 0, st>>>(p);
+    B200_SMEAR_CHECK(cudaGetLastError());
+  }
+  if (sm->nsmear > 0 && sm->lex[0]) {
+    planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(sm->lex[0], planar_level(sm, 0));
     B200_SMEAR_CHECK(cudaGetLastError());
   }
   B200_SMEAR_CHECK(cudaStreamSynchronize(st));
@@ -387,9 +473,37 @@ int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void
   return 0;
 }
 
+// A lexical copy of a level below the top, made on the first request: on a
+// stream of its own, so that a capture or work in progress on the caller's
+// streams is not touched (the levels are complete when set_config returns).
+static int make_lex(b200_smear* sm, int level) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  double* buf = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMalloc(&buf, nreal_cfg(sm) * sizeof(double));
+  if (e == cudaSuccess) {
+    planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(buf, planar_level(sm, level));
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  if (st) cudaStreamDestroy(st);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    cudaFree(buf);
+    set_last_error(e == cudaErrorMemoryAllocation ? B200_ENOMEM : B200_ECUDA, "smear_config: %s", cudaGetErrorString(e));
+    return B200_ECUDA;
+  }
+  sm->lex[level] = buf;
+  return 0;
+}
+
 const double* b200_smear_config(b200_smear_t* sm, int level) {
   if (!sm || level < 0 || level > sm->nsmear || !sm->have_config) return nullptr;
-  return sm->levels + (size_t)level * nreal_cfg(sm);
+  std::lock_guard<std::mutex> lock(sm->mu);
+  if (!sm->lex[level] && make_lex(sm, level) != 0) return nullptr;
+  return sm->lex[level];
 }
 
 int b200_smear_get_config(b200_smear_t* sm, int level, double* host_out, void* stream) {
@@ -407,21 +521,20 @@ int b200_smear_jacobian(b200_smear_t* sm, double* sigma, void* stream) {
     return B200_EINVAL;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t n = nreal_cfg(sm);
-  const int grid = (int)((4 * sm->g.vol + 127) / 128);
+  const unsigned vol = (unsigned)sm->g.vol;
   for (int i = sm->nsmear - 1; i >= 0; --i) {
-    // Sigma_i = J_i^T Sigma_(i+1): sig_tmp <- recursion(sigma), then force_each
-    B200_SMEAR_CHECK(cudaMemcpyAsync(sm->sig_tmp, sigma, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    // Sigma_i = J_i^T Sigma_(i+1): recursion, then the staple derivatives
     StoutParams p{};
-    p.u = sm->levels + (size_t)i * n;
-    p.sigp = sm->sig_tmp;
-    p.sig = sigma;
-    p.itheta = sm->itheta;
+    p.u = planar_level(sm, i);
+    p.sig = PlanarField{sm->sig, vol};
+    p.itheta = PlanarField{sm->itheta, vol};
+    if (i == sm->nsmear - 1) p.sig_in = sigma;
+    if (i == 0) p.sig_out = sigma;
     p.rho = sm->rho;
     p.g = sm->g;
-    stout_recursive_kernel<<<grid, 128, 0, st>>>(p);
+    stout_recursive_kernel<<<link_grid(sm), 128, 0, st>>>(p);
     B200_SMEAR_CHECK(cudaGetLastError());
-    stout_force_each_kernel<<<grid, 128, 0, st>>>(p);
+    stout_force_each_kernel<<<link_grid(sm), 128, 0, st>>>(p);
     B200_SMEAR_CHECK(cudaGetLastError());
   }
   return 0;
