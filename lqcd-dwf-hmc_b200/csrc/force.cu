@@ -20,6 +20,10 @@
 
 namespace b200 {
 
+// Row of a thread's 18 sums in the reduction tile, padded to an odd number of
+// doubles so that the warp's stores miss no bank.
+constexpr int kRow = 19;
+
 template <int LS, bool T1, bool T2>
 __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
   using St = Store<PREC_F64>;
@@ -27,7 +31,7 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
   constexpr int G = 32 / LS;
   constexpr int WARPS = 4;
   extern __shared__ unsigned char smem_raw[];
-  R* tile = reinterpret_cast<R*>(smem_raw) + (size_t)(threadIdx.x >> 5) * G * LS * 18;
+  R* tile = reinterpret_cast<R*>(smem_raw) + (size_t)(threadIdx.x >> 5) * G * LS * kRow;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane / LS;
   const int s = lane - g * LS;
@@ -52,45 +56,45 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
     if (T2) St::load(p.z2, vh, LS, site, s, z2);
   }
 
-#define B200_FORCE_MU(MU, COORD, EXT, NBP)                                            \
+#define B200_FORCE_MU(MU, EXT, NBP)                                                   \
   {                                                                                   \
     R f[18];                                                                          \
     _Pragma("unroll") for (int i = 0; i < 18; ++i) f[i] = 0;                          \
     if (active) {                                                                     \
-      const R ph = (COORD == EXT - 1) ? (R)p.bc[MU] : R(1);                           \
       const int nb = NBP;                                                             \
-      const R half_t = (MU == 3) ? R(0.5) : R(1);                                     \
       R w[24], h[12], gz[12];                                                         \
       if (T1) {                                                                       \
         St::load(p.y1, vh, LS, nb, s, w);                                             \
         project<R, MU, 1>(w, h);                                                      \
-        project<R, MU, 1>(z1, gz);                                                    \
+        project<R, MU, 1, false>(z1, gz);                                             \
         _Pragma("unroll") for (int a = 0; a < 2; ++a)                                 \
         _Pragma("unroll") for (int c1 = 0; c1 < 3; ++c1)                              \
         _Pragma("unroll") for (int c2 = 0; c2 < 3; ++c2) {                            \
           const R hr = h[6 * a + 2 * c1], hi = h[6 * a + 2 * c1 + 1];                 \
           const R gr = gz[6 * a + 2 * c2], gi = gz[6 * a + 2 * c2 + 1];               \
-          f[2 * (c2 + 3 * c1)] += ph * half_t * (hr * gr + hi * gi);                  \
-          f[2 * (c2 + 3 * c1) + 1] += ph * half_t * (hi * gr - hr * gi);              \
+          f[2 * (c2 + 3 * c1)] = fma(hi, gi, fma(hr, gr, f[2 * (c2 + 3 * c1)]));      \
+          f[2 * (c2 + 3 * c1) + 1] =                                                  \
+              fma(-hr, gi, fma(hi, gr, f[2 * (c2 + 3 * c1) + 1]));                    \
         }                                                                             \
       }                                                                               \
       if (T2) {                                                                       \
         St::load(p.y2, vh, LS, nb, s, w);                                             \
         project<R, MU, -1>(w, h);                                                     \
-        project<R, MU, -1>(z2, gz);                                                   \
+        project<R, MU, -1, false>(z2, gz);                                            \
         _Pragma("unroll") for (int a = 0; a < 2; ++a)                                 \
         _Pragma("unroll") for (int c1 = 0; c1 < 3; ++c1)                              \
         _Pragma("unroll") for (int c2 = 0; c2 < 3; ++c2) {                            \
           const R hr = h[6 * a + 2 * c1], hi = h[6 * a + 2 * c1 + 1];                 \
           const R gr = gz[6 * a + 2 * c2], gi = gz[6 * a + 2 * c2 + 1];               \
-          f[2 * (c2 + 3 * c1)] += ph * half_t * (hr * gr + hi * gi);                  \
-          f[2 * (c2 + 3 * c1) + 1] += ph * half_t * (hi * gr - hr * gi);              \
+          f[2 * (c2 + 3 * c1)] = fma(hi, gi, fma(hr, gr, f[2 * (c2 + 3 * c1)]));      \
+          f[2 * (c2 + 3 * c1) + 1] =                                                  \
+              fma(-hr, gi, fma(hi, gr, f[2 * (c2 + 3 * c1) + 1]));                    \
         }                                                                             \
       }                                                                               \
     }                                                                                 \
     __syncwarp();                                                                     \
     if (g < G) {                                                                      \
-      _Pragma("unroll") for (int i = 0; i < 18; ++i) tile[(g * LS + s) * 18 + i] = f[i]; \
+      _Pragma("unroll") for (int i = 0; i < 18; ++i) tile[(g * LS + s) * kRow + i] = f[i]; \
     }                                                                                 \
     __syncwarp();                                                                     \
     for (int o = lane; o < 18 * G; o += 32) {                                         \
@@ -98,31 +102,33 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
       const int st = (blockIdx.x * WARPS + warp) * G + gg;                            \
       if (st < p.vh) {                                                                \
         R sum = 0;                                                                    \
-        for (int q = 0; q < LS; ++q) sum += tile[(gg * LS + q) * 18 + i];             \
+        for (int q = 0; q < LS; ++q) sum += tile[(gg * LS + q) * kRow + i];           \
         const int sx2 = st % p.nx2, syzt = st / p.nx2;                                \
         const int sy = syzt % p.ny, sz = (syzt / p.ny) % p.nz, stt = syzt / (p.ny * p.nz); \
         const int sxx = 2 * sx2 + ((p.ieo + sy + sz + stt) & 1);                      \
+        const int coord = MU == 0 ? sxx : MU == 1 ? sy : MU == 2 ? sz : stt;          \
         const size_t lex = sxx + (size_t)(2 * p.nx2) *                                \
                            (sy + (size_t)p.ny * (sz + (size_t)p.nz * stt));           \
         double* dst = p.force + 18 * (lex + (size_t)2 * vh * MU) + i;                 \
-        *dst = (p.beta != 0.0 ? p.beta * (*dst) : 0.0) + p.coef * sum;               \
+        const R cf = coord == (EXT) - 1 ? p.coef * p.bc[MU] : p.coef;                 \
+        *dst = (p.beta != 0.0 ? p.beta * (*dst) : 0.0) + cf * sum;                    \
       }                                                                               \
     }                                                                                 \
   }
 
   const int row = p.nx2 * iyzt;
-  B200_FORCE_MU(0, x, 2 * p.nx2, row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo))
-  B200_FORCE_MU(1, y, p.ny, (y == p.ny - 1) ? site - (p.ny - 1) * p.nx2 : site + p.nx2)
+  B200_FORCE_MU(0, 2 * p.nx2, row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo))
+  B200_FORCE_MU(1, p.ny, (y == p.ny - 1) ? site - (p.ny - 1) * p.nx2 : site + p.nx2)
   const int sz_ = p.nx2 * p.ny;
-  B200_FORCE_MU(2, z, p.nz, (z == p.nz - 1) ? site - (p.nz - 1) * sz_ : site + sz_)
+  B200_FORCE_MU(2, p.nz, (z == p.nz - 1) ? site - (p.nz - 1) * sz_ : site + sz_)
   const int st_ = p.nx2 * p.ny * p.nz;
-  B200_FORCE_MU(3, t, p.nt, (t == p.nt - 1) ? site - (p.nt - 1) * st_ : site + st_)
+  B200_FORCE_MU(3, p.nt, (t == p.nt - 1) ? site - (p.nt - 1) * st_ : site + st_)
 #undef B200_FORCE_MU
 }
 
 template <int LS>
 cudaError_t run_force(const ForceParams& p, cudaStream_t st) {
-  constexpr size_t smem = sizeof(double) * 4 * (32 / LS) * LS * 18;
+  constexpr size_t smem = sizeof(double) * 4 * (32 / LS) * LS * kRow;
   const int grid = hop_grid(LS, p.vh);
   if (p.y1 && p.y2) force_kernel<LS, true, true><<<grid, 128, smem, st>>>(p);
   else if (p.y1) force_kernel<LS, true, false><<<grid, 128, smem, st>>>(p);
