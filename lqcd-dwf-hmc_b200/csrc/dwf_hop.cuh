@@ -370,7 +370,9 @@ struct HopParams {
 // With NR = 2 a block covers the sites of two one-row blocks and writes its
 // |o1|^2 partial to red[2*block] (and zero to red[2*block + 1]), so the host
 // reduces the same number of partials for either kernel shape.
-template <int LS, int P, int EPI, int FK, int NR, int GT>
+// kSolo: the caller is the only warp of its block that finishes sites; it
+// writes the block's |o1|^2 partial itself.
+template <int LS, int P, int EPI, int FK, int NR, int GT, bool kSolo = false>
 __device__ __forceinline__ void hop_epilogue_rows(const HopParams& p,
                                                   const ChainCoef<typename Store<P>::R>& k,
                                                   typename Store<P>::R (*acc)[24],
@@ -500,6 +502,10 @@ __device__ __forceinline__ void hop_epilogue_rows(const HopParams& p,
   if (p.red) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, off);
+    if (kSolo) {
+      if (lane == 0) p.red[blockIdx.x] = nrm;
+      return;
+    }
     if (lane == 0) red_warp[warp] = nrm;
     __syncthreads();
     if (tid == 0) {
@@ -524,7 +530,7 @@ __device__ __forceinline__ void hop_epilogue_rows(const HopParams& p,
   }
 }
 
-template <int LS, int P, int EPI, int FK>
+template <int LS, int P, int EPI, int FK, bool kSolo = false>
 __device__ __forceinline__ void hop_epilogue(const HopParams& p, const ChainCoef<typename Store<P>::R>& k,
                                              typename Store<P>::R* acc,
                                              typename Store<P>::R* tile, double* red_warp,
@@ -533,8 +539,8 @@ __device__ __forceinline__ void hop_epilogue(const HopParams& p, const ChainCoef
   using R = typename Store<P>::R;
   R (*rows)[24] = reinterpret_cast<R (*)[24]>(acc);
   const int srow[1] = {s};
-  hop_epilogue_rows<LS, P, EPI, FK, 1, 32 / LS>(p, k, rows, tile, red_warp, tid, lane, warp, g, srow,
-                                                site, active);
+  hop_epilogue_rows<LS, P, EPI, FK, 1, 32 / LS, kSolo>(p, k, rows, tile, red_warp, tid, lane, warp, g, srow,
+                                                       site, active);
 }
 
 // The block's streams that come from HBM rather than L2, requested at its
@@ -675,6 +681,116 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
 
   hop_epilogue<LS, P, EPI, FK>(p, k, acc, tile_all + (size_t)warp * TileWarp<R, LS, G>::v, red_warp, tid, lane,
                                warp, g, s, site, active);
+}
+
+// ---------------------------------------------------------------------------
+// Small lattices: the four hop axes on four warps.  A lattice of a few hundred
+// or thousand sites leaves most of the chip idle and every warp of the kernels
+// above walks its 8 directions one memory latency after another; here a block
+// owns the sites of one warp, warp mu fetches both neighbours along mu at once
+// and computes their two hops, the partial results meet in shared memory (a
+// quarter of the components summed by each warp) and warp 0 runs the
+// epilogue.  Kept by the autotuner where it is the fastest.  DdagD in FP64,
+// 4^3x8 Ls=8 (four hops, synchronous call): see the size rule in the plan.
+template <typename R, int P, int LS, int LF, int MU, bool kDagHop>
+__device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, int nbp, int nbm, bool lastp,
+                                           bool firstm, R* acc) {
+  using St = Store<P>;
+  constexpr bool kPh = LinkLoad<LF>::kFolded;
+  R wp[24], wm[24], up[18], um[18], h[12], o[12];
+  St::load(p.in, p.vh, LS, nbp, s, wp);
+  St::load(p.in, p.vh, LS, nbm, s, wm);
+  LinkLoad<LF>::load(p.links, (size_t)(p.ieo + 2 * MU) * p.vh + site, up);
+  LinkLoad<LF>::load(p.links, (size_t)(1 - p.ieo + 2 * MU) * p.vh + nbm, um);
+  if (kDagHop) {
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      R t = wp[q]; wp[q] = wp[q + 12]; wp[q + 12] = t;
+      t = wm[q]; wm[q] = wm[q + 12]; wm[q + 12] = t;
+    }
+  }
+  project<R, MU, 1, !kPh>(wp, h);
+  su3_mult_half<R, false>(up, h, o);
+  reconstruct_acc<R, MU, 1, kPh>(acc, o, (kPh || !lastp) ? R(1) : (R)p.bc[MU]);
+  project<R, MU, -1, !kPh>(wm, h);
+  su3_mult_half<R, true>(um, h, o);
+  reconstruct_acc<R, MU, -1, kPh>(acc, o, (kPh || !firstm) ? R(1) : (R)p.bc[MU]);
+}
+
+template <int LS, int P, int LF, int EPI, int FK>
+__global__ void __launch_bounds__(128, 2)
+dwf_hop_split_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
+  if (p.skip && *p.skip != 0.0) return;
+  using St = Store<P>;
+  using R = typename St::R;
+  constexpr bool kDagHop = EpiIsDag<EPI>::v;
+  constexpr int G = 32 / LS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  R* part = reinterpret_cast<R*>(smem_raw);            // [4 axes][24][32 lanes]; later warp 0's tile
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int g = lane / LS;
+  const int s = lane - g * LS;
+  const int site = p.site0 + blockIdx.x * G + g;
+  const bool active = (g < G) && (site < p.site_end);
+  R acc[24];
+#pragma unroll
+  for (int i = 0; i < 24; ++i) acc[i] = 0;
+  if (active) {
+    const int ix2 = site % p.nx2;
+    const int iyzt = site / p.nx2;
+    const int y = iyzt % p.ny;
+    const int izt = iyzt / p.ny;
+    const int z = izt % p.nz;
+    const int t = izt / p.nz;
+    const int keo = (p.ieo + y + z + t) & 1;
+    if (warp == 0) {
+      const int x = 2 * ix2 + keo;
+      const int row = p.nx2 * iyzt;
+      split_axis<R, P, LS, LF, 0, kDagHop>(p, s, site, row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo),
+                                           row + ((ix2 - 1 + keo < 0) ? p.nx2 - 1 : ix2 - 1 + keo),
+                                           x == 2 * p.nx2 - 1, x == 0, acc);
+    } else {
+      const int c = warp == 1 ? y : warp == 2 ? z : t;
+      const int ext = warp == 1 ? p.ny : warp == 2 ? p.nz : p.nt;
+      const int stride = warp == 1 ? p.nx2 : warp == 2 ? p.nx2 * p.ny : p.nx2 * p.ny * p.nz;
+      const bool lastp = c == ext - 1, firstm = c == 0;
+      const int nbp = lastp ? site - (ext - 1) * stride : site + stride;
+      const int nbm = firstm ? site + (ext - 1) * stride : site - stride;
+      if (warp == 1) split_axis<R, P, LS, LF, 1, kDagHop>(p, s, site, nbp, nbm, lastp, firstm, acc);
+      else if (warp == 2) split_axis<R, P, LS, LF, 2, kDagHop>(p, s, site, nbp, nbm, lastp, firstm, acc);
+      else split_axis<R, P, LS, LF, 3, kDagHop>(p, s, site, nbp, nbm, lastp, firstm, acc);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 24; ++i) part[(warp * 24 + i) * 32 + lane] = acc[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    R* q = part + (warp * 6 + i) * 32 + lane;
+    const R a = q[0], b = q[24 * 32], c = q[2 * 24 * 32], d = q[3 * 24 * 32];
+    q[0] = (a + b) + (c + d);
+  }
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int i = 0; i < 24; ++i) acc[i] = part[i * 32 + lane];
+  __syncwarp();
+  hop_epilogue<LS, P, EPI, FK, true>(p, k, acc, part, nullptr, tid, lane, 0, g, s, site, active);
+}
+
+template <int LS, int P>
+constexpr size_t hop_split_smem_bytes() {
+  using R = typename Store<P>::R;
+  constexpr size_t tile = sizeof(R) * TileWarp<R, LS, 32 / LS>::v;
+  return sizeof(R) * 4 * 24 * 32 > tile ? sizeof(R) * 4 * 24 * 32 : tile;
+}
+
+// Blocks of the split kernel: the sites of one warp each.
+inline int hop_split_grid(int ls, int vh) {
+  const int g = 32 / ls;
+  return (vh + g - 1) / g;
 }
 
 // ---------------------------------------------------------------------------

@@ -130,6 +130,8 @@ cudaError_t launch_force(const ForceParams& p, cudaStream_t st);
 
 // number of blocks the reductions of each launcher produce
 int hop_grid(int ls, int vh);
+constexpr int kHopSplit = 10;   // the hop variant whose blocks hold one warp's sites
+int hop_partials(int variant, int ls, int vh);   // |o1|^2 partials of a hop launch
 int site_s_grid(int ls, int vh);
 constexpr int kSiteSBlock = 128;
 

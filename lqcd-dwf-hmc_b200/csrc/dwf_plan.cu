@@ -269,12 +269,19 @@ SopParams sop_base(const b200_dwf* op) {
 // B200_AUTOTUNE=0 disables tuning (variant 0).  The first call of a
 // combination must not be inside a CUDA graph capture.
 typedef std::tuple<int, int, int, int, int> TuneKey;   // vh, ls, prec, epi, fk
-constexpr int kHopVariants = 10;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
+constexpr int kHopVariants = 11;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
                                   // higher occupancy, packed two-slice FP32x2 (direct, TMA),
                                   // 4-deep TMA, packed with all directions in flight, packed
-                                  // half-storage with register prefetch
+                                  // half-storage with register prefetch, the four axes on
+                                  // four warps
+// Above this many sites every SM has several blocks of the other variants and
+// the split kernel's extra pass through shared memory only costs (FP64 D_eo
+// at 16^3x32, 65,536 sites: it is the slowest of the variants); its block
+// partials fit the plan's buffer up to here.
+constexpr int kSplitMaxSites = 16384;
 
-bool variant_supported(int prec, int ls, int v) {
+bool variant_supported(int prec, int ls, int vh, int v) {
+  if (v == kHopSplit) return vh <= kSplitMaxSites;
   if (v < 5) return true;
   if (v == 7 && prec == PREC_F64) return true;
   if (v == 9 && (prec == PREC_F64 || prec == PREC_F32)) return false;
@@ -319,7 +326,7 @@ int tune_hop(b200_dwf* op, int prec, const HopParams& p0, cudaStream_t st, int* 
   float t[kHopVariants];
   int nv = 0;
   for (int v = 0; v < kHopVariants; ++v)
-    if (variant_supported(prec, op->g.ls, v)) { vs[nv] = v; t[nv] = 1e30f; ++nv; }
+    if (variant_supported(prec, op->g.ls, op->g.vh, v)) { vs[nv] = v; t[nv] = 1e30f; ++nv; }
   for (int i = 0; i < nv; ++i) {     // first launches: module loads, first touches
     p.variant = vs[i];
     B200_CHECK_CUDA(launch_hop(prec, p, op->coefs, st));
@@ -388,7 +395,7 @@ static int no_halo(const b200_dwf* op, const char* what) {
 static int select_variant(b200_dwf* op, int prec, HopParams& p, cudaStream_t st) {
   int variant = 0;
   const int fv = forced_variant();
-  if (fv >= 0 && variant_supported(prec, op->g.ls, fv)) {
+  if (fv >= 0 && variant_supported(prec, op->g.ls, op->g.vh, fv)) {
     variant = fv;
   } else if (tuning_enabled()) {
     const TuneKey key(op->g.vh, op->g.ls, prec, p.epi, p.fk);
@@ -707,7 +714,8 @@ int b200_dwf_create(b200_dwf_t** out, const int lattice[4], int Ls, double mq, d
       op->coefs.dee_f.wc2[s] = (float)op->coefs.dee_d.wc2[s];
     }
   }
-  const int red_n = site_s_grid(Ls, op->g.vh) + hop_grid(Ls, op->g.vh);
+  int red_n = site_s_grid(Ls, op->g.vh) + hop_grid(Ls, op->g.vh);
+  if (op->g.vh <= kSplitMaxSites) red_n += hop_partials(kHopSplit, Ls, op->g.vh);
   op->red_n = red_n;
   if (cudaMalloc(&op->red, (size_t)red_n * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&op->sc, SC_N * sizeof(double)) != cudaSuccess ||
@@ -1013,7 +1021,7 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
     p2.out2 = u;
     p2.red = op->red;
     if ((rc = run_hop(op, prec, p2, st))) return rc;
-    if ((rc = reduce_to(op, nb_hop, op->sc, FIN_CG_ALPHA, st))) return rc;
+    if ((rc = reduce_to(op, hop_partials(p2.variant, g.ls, g.vh), op->sc, FIN_CG_ALPHA, st))) return rc;
 
     HopParams p3 = hop_base(op, prec, 1, EPI_K3);
     p3.in = u; p3.out1 = t3;
@@ -1026,7 +1034,7 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
     p4.x2 = t2; p4.c_x2 = -1.0; p4.c_x2_dev = op->sc + SC_ALPHA;
     p4.red = op->red;
     if ((rc = run_hop(op, prec, p4, st))) return rc;
-    if ((rc = reduce_to(op, nb_hop, op->sc, FIN_CG_BETA, st))) return rc;
+    if ((rc = reduce_to(op, hop_partials(p4.variant, g.ls, g.vh), op->sc, FIN_CG_BETA, st))) return rc;
 
     CgUpdParams pu;
     pu.x = x; pu.p = p; pu.r = r; pu.y = op->m5pre_id ? nullptr : yp;
@@ -1239,7 +1247,7 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
     p2.in = y1; p2.out1 = t2; p2.x1 = p0; p2.c_x1 = 1.0; p2.out2 = u; p2.red = op->red;
     p2.skip = S + MS_DONE;
     if ((rc2 = run_hop(op, prec, p2, s))) return rc2;
-    B200_CHECK_CUDA(launch_ms_scalar(MSS_BETA, op->red, nb_hop, S, nshift, s));
+    B200_CHECK_CUDA(launch_ms_scalar(MSS_BETA, op->red, hop_partials(p2.variant, g.ls, g.vh), S, nshift, s));
     HopParams p3 = hop_base(op, prec, 1, EPI_K3);
     p3.in = u; p3.out1 = t3; p3.skip = S + MS_DONE;
     if ((rc2 = run_hop(op, prec, p3, s))) return rc2;
@@ -1252,7 +1260,7 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
     p4.x3 = p0; p4.c_x3 = sigma[0]; p4.c_x3_dev = S + MS_BETA;
     p4.red = op->red; p4.skip = S + MS_DONE;
     if ((rc2 = run_hop(op, prec, p4, s))) return rc2;
-    B200_CHECK_CUDA(launch_ms_scalar(MSS_ALPHA, op->red, nb_hop, S, nshift, s));
+    B200_CHECK_CUDA(launch_ms_scalar(MSS_ALPHA, op->red, hop_partials(p4.variant, g.ls, g.vh), S, nshift, s));
     MsUpdParams mu;
     mu.xs = op->ms_ptrs; mu.ps = op->ms_ptrs + kMaxShift; mu.r = r; mu.y0 = op->m5pre_id ? nullptr : y0;
     mu.st = S; mu.red = op->ms_red; mu.nblocks = nb_hop; mu.g = g;

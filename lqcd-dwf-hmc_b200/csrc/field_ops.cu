@@ -18,6 +18,10 @@ int hop_grid(int ls, int vh) {
   return (vh + per_block - 1) / per_block;
 }
 
+int hop_partials(int variant, int ls, int vh) {
+  return variant == kHopSplit ? hop_split_grid(ls, vh) : hop_grid(ls, vh);
+}
+
 int site_s_grid(int ls, int vh) {
   const long n = (long)vh * ls;
   return (int)((n + kSiteSBlock - 1) / kSiteSBlock);

@@ -105,6 +105,24 @@ cudaError_t run_tma_pair(const HopParams& p, const ChainCoefs& c, cudaStream_t s
   return cudaGetLastError();
 }
 
+template <int LS, int P, int EPI, int FK>
+cudaError_t run_split(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
+  using R = typename Store<P>::R;
+  constexpr int LF = DefaultLink<P>::v;
+  constexpr size_t smem = hop_split_smem_bytes<LS, P>();
+  auto k = dwf_hop_split_kernel<LS, P, LF, EPI, FK>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr_done = true;
+  }
+  const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
+      std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
+  k<<<hop_split_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
+  return cudaGetLastError();
+}
+
 // variant 0: direct loads; 1: TMA-staged, 2 stages; 2: TMA-staged, 3 stages;
 // 3: TMA-staged, 2 stages, register budget for HopMinBlocks::v1 resident
 // blocks; 4: direct loads with that register budget; 5: packed FP32x2 kernel,
@@ -113,9 +131,11 @@ cudaError_t run_tma_pair(const HopParams& p, const ChainCoefs& c, cudaStream_t s
 // arithmetic: the packed kernel) at 2 resident blocks; 8: the packed kernel
 // with all 8 directions in flight at once; 9: the packed kernel for f16/bf16
 // storage fetching the next direction into registers while computing the
-// current one (5-9 packed: FP32 arithmetic only).
+// current one (5-9 packed: FP32 arithmetic only); 10: the four axes on four
+// warps, for small lattices.
 template <int LS, int P, int EPI, int FK>
 cudaError_t run(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
+  if (p.variant == kHopSplit) return run_split<LS, P, EPI, FK>(p, c, st);
   if (p.variant == 1) return run_tma<LS, P, EPI, FK, 2, 1>(p, c, st);
   if (p.variant == 2) return run_tma<LS, P, EPI, FK, 3, 1>(p, c, st);
   if (p.variant == 3) return run_tma<LS, P, EPI, FK, 2, HopMinBlocks<P>::v1>(p, c, st);
