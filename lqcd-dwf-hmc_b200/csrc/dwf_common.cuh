@@ -30,6 +30,16 @@ enum Prec { PREC_F64 = 0, PREC_F32 = 1, PREC_F16 = 2, PREC_BF16 = 3 };
 
 constexpr int kMaxLs = 32;
 
+// ---------------------------------------------------------------- launch overlap
+// The kernels of an operator application or a solver iteration follow one
+// another on the same fields, and on small lattices the launch and first
+// instructions of each took a quarter of its time.  A kernel first lets the
+// next one launch, does what depends on its parameters alone (index
+// arithmetic, L2 requests for the links), and waits here for the kernels
+// before it to have finished and their writes to be visible.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- storage
 template <int P> struct Store;
 

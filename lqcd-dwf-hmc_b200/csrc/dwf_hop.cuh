@@ -589,8 +589,10 @@ template <> struct HopMinBlocks<PREC_BF16> { static constexpr int v0 = 4, v1 = 6
 template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  if (p.skip && *p.skip != 0.0) return;
+  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), true);
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
   constexpr bool kDagHop = EpiIsDag<EPI>::v;
@@ -720,6 +722,8 @@ __device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, 
 template <int LS, int P, int LF, int EPI, int FK>
 __global__ void __launch_bounds__(128, 2)
 dwf_hop_split_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -875,8 +879,10 @@ __device__ __forceinline__ void reconstruct_acc2(float2* acc, const float2* o, f
 template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_pair_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  if (p.skip && *p.skip != 0.0) return;
+  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), true);
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
   static_assert(sizeof(R) == 4, "packed kernel is for FP32 arithmetic");
@@ -1107,8 +1113,10 @@ __device__ __forceinline__ void pair_compute(const PairRaw<P>& r, float ph, floa
 template <int LS, int P, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_pair_pf_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  if (p.skip && *p.skip != 0.0) return;
+  pdl_launch_dependents();
   hop_prefetch<LS, P, LINK_F16_18>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), true);
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
   static_assert(St::kScaled, "prefetching packed kernel is for f16/bf16 storage");
@@ -1244,8 +1252,10 @@ template <int LS, int P, int LF, int GS = 32 / LS> struct TmaGeom {
 template <int LS, int P, int LF, int EPI, int FK, int S, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_tma_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  if (p.skip && *p.skip != 0.0) return;
+  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), false);
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
   using TG = TmaGeom<LS, P, LF>;
@@ -1416,8 +1426,10 @@ dwf_hop_tma_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename
 template <int LS, int P, int LF, int EPI, int FK, int S, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_tma_pair_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  if (p.skip && *p.skip != 0.0) return;
+  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), false);
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
   static_assert(sizeof(R) == 4, "packed kernel is for FP32 arithmetic");

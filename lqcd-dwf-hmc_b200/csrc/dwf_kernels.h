@@ -49,6 +49,7 @@ struct CgUpdParams {
   void* y;               // M5pre(p) for the next hop; null when M5pre is the identity
   const double* alpha;
   const double* beta;
+  const double* done;    // SC_DONE: the update of a finished solve does nothing
   Geom g;
 };
 
@@ -128,6 +129,24 @@ struct ForceParams {
 };
 cudaError_t launch_force(const ForceParams& p, cudaStream_t st);
 
+// Launch with programmatic stream serialisation: the kernel may start while
+// the one before it in the stream drains; it runs pdl_wait() (dwf_common.cuh)
+// before it touches anything an earlier kernel wrote or reads.
+template <typename... KA, typename... A>
+cudaError_t launch_pdl(void (*kernel)(KA...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // number of blocks the reductions of each launcher produce
 int hop_grid(int ls, int vh);
 constexpr int kHopSplit = 10;   // the hop variant whose blocks hold one warp's sites
@@ -167,9 +186,17 @@ cudaError_t launch_links_from_lex(int lf, void* out, const double* u_lex_dev, co
 enum FinalizeOp {
   FIN_SUM = 0,          // out[0] = s
   FIN_CG_ALPHA = 1,     // sc[PQ] = s; sc[ALPHA] = sc[RR] / s
-  FIN_CG_BETA = 2,      // sc[BETA] = s / sc[RR]; sc[RR] = s
+  FIN_CG_BETA = 2,      // sc[BETA] = s / sc[RR]; sc[RR] = s; counts the iteration, decides the stop
 };
-enum CgScalar { SC_RR = 0, SC_PQ = 1, SC_ALPHA = 2, SC_BETA = 3, SC_RR_NEW = 4, SC_N = 8 };
+// SC_DONE: 0 while a CG iterates; 1 from the scalar step that met the stopping
+// rule (its x, p update still runs), 2 from the next iteration's first scalar
+// step on, 3 after a NaN.  The kernels of iterations queued past the end skip
+// themselves on it, so the host need not read every iteration's residual
+// before it queues the next.
+enum CgScalar {
+  SC_RR = 0, SC_PQ = 1, SC_ALPHA = 2, SC_BETA = 3, SC_RR_NEW = 4,
+  SC_DONE = 5, SC_ITER = 6, SC_BNORM = 7, SC_TOL2 = 8, SC_N = 10
+};
 cudaError_t launch_finalize(const double* partials, int n, double* out, int op, cudaStream_t st);
 
 size_t link_bytes(int lf, size_t vh);

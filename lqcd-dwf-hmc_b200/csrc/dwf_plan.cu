@@ -163,6 +163,10 @@ struct b200_dwf {
   double* sc = nullptr;         // solver scalars (device)
   double* sc_host = nullptr;    // pinned mirror (also of the multishift scalars)
   int* err_host = nullptr;      // pinned mirror of err
+  // two pinned snapshots of (scalars, error word) of a CG in progress, and
+  // the events that say they have arrived
+  double* cg_host = nullptr;
+  cudaEvent_t cg_ev[2] = {};
   bool async_calls = false;     // mult / force return without synchronising (b200_dwf_set_async)
   b200_halo_fn halo_fn = nullptr;   // fills (or starts filling) a field's ghost t-slices
   b200_halo_fn halo_finish = nullptr;  // with the split hooks: waits for that filling
@@ -742,6 +746,9 @@ int b200_dwf_destroy(b200_dwf_t* op) {
   cudaFree(op->err);
   if (op->sc_host) cudaFreeHost(op->sc_host);
   if (op->err_host) cudaFreeHost(op->err_host);
+  if (op->cg_host) cudaFreeHost(op->cg_host);
+  for (int i = 0; i < 2; ++i)
+    if (op->cg_ev[i]) cudaEventDestroy(op->cg_ev[i]);
   cudaFree(op->stage);
   for (int d = 0; d < 2; ++d)
     for (int k = 0; k < 2; ++k) {
@@ -972,9 +979,14 @@ int b200_field_copy_convert(b200_dwf_t* op, int prec_out, void* out, int prec_in
 //   K3 t3 = LUdag M5^+ (-1/2 g5) hop^+(u)
 //   K4 r  = r - alpha*(t2 - M5^+(-1/2 g5) hop^+(t3)) = r - alpha DdagD p ; rr
 //   K5 x += alpha p ; p = r + beta p ; yp = M5pre p
-// Scalars stay on the device; the host reads |r|^2 once per iteration for the
-// stopping test.  Returns the iteration count in *nconv and |r|^2/|b|^2 of the
-// recursive residual in *rel2.
+// Scalars and the stop decision stay on the device (SC_DONE): the host queues
+// kCgBlock iterations at a time and reads the state of the block before the
+// one it has just queued, so the device never waits for the host (8^4 Ls=12
+// FP64: one read and wait per iteration was 25 of its 72 us); what is queued
+// past the last iteration does nothing.  Returns the iteration count in
+// *nconv and |r|^2/|b|^2 of the recursive residual in *rel2.
+constexpr int kCgBlock = 2;
+
 struct CgSnap {
   int n;                 // number of snapshots
   const int* iters;      // iteration after which x is copied
@@ -995,7 +1007,6 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
   void* r = op->work[5][prec];
   void* p = op->work[6][prec];
   const Geom& g = op->g;
-  const int nb_hop = hop_grid(g.ls, g.vh);
 
   B200_CHECK_CUDA(launch_axpby(prec, g, r, b, 1.0, nullptr, 0.0, nullptr, st));
   B200_CHECK_CUDA(launch_axpby(prec, g, p, b, 1.0, nullptr, 0.0, nullptr, st));
@@ -1009,22 +1020,30 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
   if (op->m5pre_id) yp = p;
   else if ((rc = apply_sop(op, prec, yp, p, SOP_M5PRE, st))) return rc;
 
-  double rr = bnorm2;
-  for (int it = 0; it < maxiter; ++it) {
+  if (!op->cg_host &&
+      cudaMallocHost(&op->cg_host, 2 * (SC_N + 1) * sizeof(double)) != cudaSuccess)
+    return fail(B200_ENOMEM, "page-locked allocation for the CG state failed");
+  for (int i = 0; i < 2; ++i)
+    if (!op->cg_ev[i]) B200_CHECK_CUDA(cudaEventCreateWithFlags(&op->cg_ev[i], cudaEventDisableTiming));
+  const double start[4] = {0.0, 0.0, bnorm2, tol2};    // SC_DONE, SC_ITER, SC_BNORM, SC_TOL2
+  B200_CHECK_CUDA(cudaMemcpyAsync(op->sc + SC_DONE, start, sizeof(start), cudaMemcpyHostToDevice, st));
+  const double* done = op->sc + SC_DONE;
+
+  auto iteration = [&](int it) -> int {
     HopParams p1 = hop_base(op, prec, 1, EPI_K1);
-    p1.in = yp; p1.out1 = y1;
+    p1.in = yp; p1.out1 = y1; p1.skip = done;
     if ((rc = run_hop(op, prec, p1, st))) return rc;
 
     HopParams p2 = hop_base(op, prec, 0, EPI_K2N, F_LUDAG);
     p2.in = y1; p2.out1 = t2;
     p2.x1 = p; p2.c_x1 = 1.0;
     p2.out2 = u;
-    p2.red = op->red;
+    p2.red = op->red; p2.skip = done;
     if ((rc = run_hop(op, prec, p2, st))) return rc;
     if ((rc = reduce_to(op, hop_partials(p2.variant, g.ls, g.vh), op->sc, FIN_CG_ALPHA, st))) return rc;
 
     HopParams p3 = hop_base(op, prec, 1, EPI_K3);
-    p3.in = u; p3.out1 = t3;
+    p3.in = u; p3.out1 = t3; p3.skip = done;
     if ((rc = run_hop(op, prec, p3, st))) return rc;
 
     HopParams p4 = hop_base(op, prec, 0, EPI_K4N);
@@ -1032,25 +1051,49 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
     p4.ce = -1.0; p4.ce_dev = op->sc + SC_ALPHA;
     p4.x1 = r; p4.c_x1 = 1.0;
     p4.x2 = t2; p4.c_x2 = -1.0; p4.c_x2_dev = op->sc + SC_ALPHA;
-    p4.red = op->red;
+    p4.red = op->red; p4.skip = done;
     if ((rc = run_hop(op, prec, p4, st))) return rc;
     if ((rc = reduce_to(op, hop_partials(p4.variant, g.ls, g.vh), op->sc, FIN_CG_BETA, st))) return rc;
 
     CgUpdParams pu;
     pu.x = x; pu.p = p; pu.r = r; pu.y = op->m5pre_id ? nullptr : yp;
-    pu.alpha = op->sc + SC_ALPHA; pu.beta = op->sc + SC_BETA; pu.g = g;
+    pu.alpha = op->sc + SC_ALPHA; pu.beta = op->sc + SC_BETA; pu.done = done; pu.g = g;
     B200_CHECK_CUDA(launch_cg_update(prec, pu, op->coefs, st));
     if (snap)
       for (int j = 0; j < snap->n; ++j)
         if (snap->iters[j] == it + 1)
           B200_CHECK_CUDA(cudaMemcpyAsync(snap->dst[j], x, field_bytes(prec, g.vh, g.ls),
                                           cudaMemcpyDeviceToDevice, st));
-
-    if ((rc = host_scalar(op, SC_RR, &rr, st))) return rc;
-    *nconv = it + 1;
-    if (!(rr == rr)) return fail(B200_ENOCONV, "CG breakdown: residual is NaN at iteration %d", it + 1);
-    if (rr / bnorm2 < tol2) break;
+    return 0;
+  };
+  // snapshots are copies after a given iteration, so with them every
+  // iteration's outcome is read before the next is queued
+  const int block = snap ? 1 : kCgBlock;
+  double rr = bnorm2;
+  bool over = false;
+  for (int it = 0, b2 = 0; it < maxiter && !over; ++b2) {
+    for (int k = 0; k < block && it < maxiter; ++k, ++it)
+      if ((rc = iteration(it))) return rc;
+    double* slot = op->cg_host + (b2 & 1) * (SC_N + 1);
+    B200_CHECK_CUDA(cudaMemcpyAsync(slot, op->sc, SC_N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    B200_CHECK_CUDA(cudaMemcpyAsync(slot + SC_N, op->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    B200_CHECK_CUDA(cudaEventRecord(op->cg_ev[b2 & 1], st));
+    // the block before this one, then (no more to queue) this one
+    for (int c = (snap || b2 == 0) ? b2 : b2 - 1; c <= b2 && !over; ++c) {
+      if (c == b2 && !snap && it < maxiter) break;
+      B200_CHECK_CUDA(cudaEventSynchronize(op->cg_ev[c & 1]));
+      const double* s = op->cg_host + (c & 1) * (SC_N + 1);
+      memcpy(op->err_host, s + SC_N, sizeof(int));
+      if (*op->err_host != 0) {
+        B200_CHECK_CUDA(cudaStreamSynchronize(st));
+        return report_err(op, st);
+      }
+      rr = s[SC_RR];
+      *nconv = (int)s[SC_ITER];
+      over = s[SC_DONE] != 0.0;
+    }
   }
+  if (!(rr == rr)) return fail(B200_ENOCONV, "CG breakdown: residual is NaN at iteration %d", *nconv);
   *rel2 = rr / bnorm2;
   if (!(rr / bnorm2 < tol2))
     return fail(B200_ENOCONV, "CG not converged in %d iterations: |r|^2/|b|^2 = %.3e", maxiter,

@@ -84,6 +84,8 @@ template <int LS, int P, int OPA, int OPB>
 __global__ void __launch_bounds__(128)
 sop_kernel(SopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k,
            const __grid_constant__ ChainCoef<typename Store<P>::R> kee) {
+  pdl_launch_dependents();
+  pdl_wait();
   using St = Store<P>;
   using R = typename St::R;
   constexpr int G = 32 / LS;
@@ -176,8 +178,7 @@ cudaError_t run_sop(const SopParams& p, const ChainCoefs& c, cudaStream_t st) {
   const bool dbl = std::is_same<R, double>::value;
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(dbl ? (const void*)&c.d : (const void*)&c.f);
   const ChainCoef<R>& ke = *reinterpret_cast<const ChainCoef<R>*>(dbl ? (const void*)&c.dee_d : (const void*)&c.dee_f);
-  k<<<hop_grid(LS, p.g.vh), 128, smem, st>>>(p, kc, ke);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_grid(LS, p.g.vh), 128, smem, st, p, kc, ke);
 }
 
 template <int LS, int P>
@@ -227,6 +228,9 @@ cudaError_t launch_sop(int prec, const SopParams& p, const ChainCoefs& c, cudaSt
 template <int LS, int P>
 __global__ void __launch_bounds__(128)
 cg_update_kernel(CgUpdParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (*p.done >= 2.0) return;
   using St = Store<P>;
   using R = typename St::R;
   constexpr int G = 32 / LS;
@@ -288,8 +292,7 @@ cudaError_t run_cgu(const CgUpdParams& p, const ChainCoefs& c, cudaStream_t st) 
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
       std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
-  k<<<hop_grid(LS, p.g.vh), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_grid(LS, p.g.vh), 128, smem, st, p, kc);
 }
 
 template <int P>
@@ -323,6 +326,8 @@ __global__ void __launch_bounds__(128)
 ms_update_kernel(MsUpdParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
   using St = Store<P>;
   using R = typename St::R;
+  pdl_launch_dependents();
+  pdl_wait();
   if (p.st[MS_DONE] != 0.0) return;   // solve finished: replayed iteration is a no-op
   constexpr int G = 32 / LS;
   constexpr int WARPS = 4;
@@ -416,8 +421,7 @@ cudaError_t run_msu(const MsUpdParams& p, const ChainCoefs& c, cudaStream_t st) 
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
       std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
-  k<<<hop_grid(LS, p.g.vh), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_grid(LS, p.g.vh), 128, smem, st, p, kc);
 }
 
 template <int P>
@@ -459,6 +463,8 @@ __device__ double block_sum_partials(const double* partials, int n) {
 }
 
 __global__ void ms_scalar_kernel(int step, const double* partials, int n, double* st, int nshift) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (st[MS_DONE] != 0.0) return;     // solve finished: a replayed iteration is a no-op
   double* zeta1 = st + MS_N + MSA_ZETA1 * kMaxShift;
   double* zeta2 = st + MS_N + MSA_ZETA2 * kMaxShift;
@@ -549,8 +555,7 @@ __global__ void ms_scalar_kernel(int step, const double* partials, int n, double
 
 cudaError_t launch_ms_scalar(int step, const double* partials, int n, double* st, int nshift,
                              cudaStream_t stream) {
-  ms_scalar_kernel<<<1, 1024, 0, stream>>>(step, partials, n, st, nshift);
-  return cudaGetLastError();
+  return launch_pdl(ms_scalar_kernel, 1, 1024, 0, stream, step, partials, n, st, nshift);
 }
 
 // Windowed multishift: the window is applied when it is full or when the
@@ -563,6 +568,8 @@ __device__ __forceinline__ bool ms_window_due(const double* st) {
 // p_i = PC0 p_i + sum_l PC_l r_l ; x_i += XC0 p_i(old) + sum_l XC_l r_l for
 // every shift active in the window; flat over the FP64 field as double2.
 __global__ void __launch_bounds__(256) ms_flush_kernel(MsUpdParams p, long n2) {
+  pdl_launch_dependents();
+  pdl_wait();
   const double* st = p.st;
   if (!ms_window_due(st)) return;
   __shared__ double cs[2 * kMaxShift * (kMaxWin + 1)];
@@ -627,6 +634,8 @@ __global__ void __launch_bounds__(256) ms_flush_kernel(MsUpdParams p, long n2) {
 }
 
 __global__ void ms_window_reset_kernel(double* st) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (threadIdx.x != 0 || !ms_window_due(st)) return;
   for (int i = 0; i < kMaxShift; ++i) {
     double* pc = st + kMsCoef + i * (kMaxWin + 1);
@@ -642,13 +651,11 @@ cudaError_t launch_ms_flush(const MsUpdParams& p, cudaStream_t st) {
   const long n2 = (long)12 * p.g.vh * p.g.ls;      // FP64 field as double2
   long blocks = (n2 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  ms_flush_kernel<<<(int)blocks, 256, 0, st>>>(p, n2);
-  return cudaGetLastError();
+  return launch_pdl(ms_flush_kernel, (int)blocks, 256, 0, st, p, n2);
 }
 
 cudaError_t launch_ms_window_reset(double* st, cudaStream_t stream) {
-  ms_window_reset_kernel<<<1, 32, 0, stream>>>(st);
-  return cudaGetLastError();
+  return launch_pdl(ms_window_reset_kernel, 1, 32, 0, stream, st);
 }
 
 // ------------------------------------------------------------ BLAS
@@ -834,7 +841,13 @@ size_t link_bytes(int lf, size_t vh) {
 }
 
 __global__ void finalize_kernel(const double* partials, int n, double* out, int op) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ double ws[32];
+  if (op != FIN_SUM && out[SC_DONE] != 0.0) {       // a CG that is over
+    if (threadIdx.x == 0 && op == FIN_CG_ALPHA && out[SC_DONE] == 1.0) out[SC_DONE] = 2.0;
+    return;
+  }
   double v = 0.0;
   // fixed assignment of partials to threads -> deterministic result
   for (int i = threadIdx.x; i < n; i += blockDim.x) v += partials[i];
@@ -853,6 +866,9 @@ __global__ void finalize_kernel(const double* partials, int n, double* out, int 
     } else if (op == FIN_CG_BETA) {
       out[SC_BETA] = s / out[SC_RR];
       out[SC_RR] = s;
+      out[SC_ITER] += 1.0;
+      if (!(s == s)) out[SC_DONE] = 3.0;
+      else if (s / out[SC_BNORM] < out[SC_TOL2]) out[SC_DONE] = 1.0;
     }
   }
 }
@@ -949,8 +965,7 @@ cudaError_t launch_links_from_lex(int lf, void* out, const double* u_lex_dev, co
 }
 
 cudaError_t launch_finalize(const double* partials, int n, double* out, int op, cudaStream_t st) {
-  finalize_kernel<<<1, 1024, 0, st>>>(partials, n, out, op);
-  return cudaGetLastError();
+  return launch_pdl(finalize_kernel, 1, 1024, 0, st, partials, n, out, op);
 }
 
 // ------------------------------------------------------------ complex BLAS (f64)

@@ -33,8 +33,7 @@ cudaError_t run_mb(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
       std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
-  k<<<hop_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 template <int LS, int P, int EPI, int FK, int S, int MB>
@@ -51,8 +50,7 @@ cudaError_t run_tma(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
       std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
-  k<<<hop_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 template <int LS, int P, int EPI, int FK>
@@ -68,8 +66,7 @@ cudaError_t run_pair(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
     attr_done = true;
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(&c.f);
-  k<<<hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 template <int LS, int P, int EPI, int FK>
@@ -84,8 +81,7 @@ cudaError_t run_pair_pf(const HopParams& p, const ChainCoefs& c, cudaStream_t st
     attr_done = true;
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(&c.f);
-  k<<<hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 template <int LS, int P, int EPI, int FK, int S, int MB>
@@ -101,8 +97,7 @@ cudaError_t run_tma_pair(const HopParams& p, const ChainCoefs& c, cudaStream_t s
     attr_done = true;
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(&c.f);
-  k<<<hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 template <int LS, int P, int EPI, int FK>
@@ -119,8 +114,7 @@ cudaError_t run_split(const HopParams& p, const ChainCoefs& c, cudaStream_t st) 
   }
   const ChainCoef<R>& kc = *reinterpret_cast<const ChainCoef<R>*>(
       std::is_same<R, double>::value ? (const void*)&c.d : (const void*)&c.f);
-  k<<<hop_split_grid(LS, p.site_end - p.site0), 128, smem, st>>>(p, kc);
-  return cudaGetLastError();
+  return launch_pdl(k, hop_split_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
 // variant 0: direct loads; 1: TMA-staged, 2 stages; 2: TMA-staged, 3 stages;
