@@ -586,102 +586,147 @@ template <> struct HopMinBlocks<PREC_F32> { static constexpr int v0 = 4, v1 = 6;
 template <> struct HopMinBlocks<PREC_F16> { static constexpr int v0 = 4, v1 = 6; };
 template <> struct HopMinBlocks<PREC_BF16> { static constexpr int v0 = 4, v1 = 6; };
 
+// A warp's link records in shared memory (full FP64 records).  A broadcast
+// 16-byte load of a link costs the L1 data pipe five of its cycles from global
+// memory and under three from shared memory; with nine of them per direction
+// they were over a third of the direct hop's L1 work, which at 77 % busy
+// bounded it.  The warp fetches the 8 records of each of its G sites at its
+// start, whole lines at a time.  FP64, with the budget of 4 resident blocks now
+// almost free of spills: force 24^3x48 Ls=16 (three hops of 5.5 ms) 5.50 ->
+// 5.21 ms, DdagD Moebius 14x10x6x18 Ls=12 116.8 -> 104.3 us.
+template <int LS, int LF> struct LinkStage {
+  static constexpr bool on = LF == LINK_F64_18;
+  static constexpr int G = 32 / LS;
+  static constexpr int records = G * 8;
+  static constexpr int bytes = on ? records * (144 + 4) : 0;       // records, then their indices
+};
+
+// Bytes of shared memory per warp of the direct kernel: the staged links and,
+// after them, the epilogue's tile in the same place.
+template <int LS, int P, int LF>
+constexpr int hop_direct_warp_bytes() {
+  using R = typename Store<P>::R;
+  constexpr int tile = TileWarp<R, LS, 32 / LS>::v * (int)sizeof(R);
+  constexpr int v = tile > LinkStage<LS, LF>::bytes ? tile : LinkStage<LS, LF>::bytes;
+  return (v + 15) / 16 * 16;
+}
+
 template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
+  using LSt = LinkStage<LS, LF>;
   pdl_launch_dependents();
-  hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), true);
-  pdl_wait();
-  if (p.skip && *p.skip != 0.0) return;
+  hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), !LSt::on);
   using St = Store<P>;
   using R = typename St::R;
   constexpr bool kDagHop = EpiIsDag<EPI>::v;
   constexpr bool kPh = LinkLoad<LF>::kFolded;
   constexpr int G = 32 / LS;              // sites per warp
   constexpr int WARPS = 4;
-  constexpr bool kTile = (EPI != EPI_HALF) || (FK != F_NONE);
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* tile_all = reinterpret_cast<R*>(smem_raw);        // WARPS * TileWarp
   __shared__ double red_warp[WARPS];
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
+  unsigned char* wbase = smem_raw + (size_t)warp * hop_direct_warp_bytes<LS, P, LF>();
   const int g = lane / LS;
   const int s = lane - g * LS;
   const int site = p.site0 + (blockIdx.x * WARPS + warp) * G + g;
   const bool active = (g < G) && (site < p.site_end);
   const size_t vh = p.vh;
 
-  R acc[24];
-#pragma unroll
-  for (int i = 0; i < 24; ++i) acc[i] = 0;
-
+  int nb[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // neighbours x+, x-, y+, ..., t-
+  int x = 0, y = 0, z = 0, t = 0;
   if (active) {
     const int ix2 = site % p.nx2;
     const int iyzt = site / p.nx2;
-    const int y = iyzt % p.ny;
+    y = iyzt % p.ny;
     const int izt = iyzt / p.ny;
-    const int z = izt % p.nz;
-    const int t = izt / p.nz;
+    z = izt % p.nz;
+    t = izt / p.nz;
     const int keo = (p.ieo + y + z + t) & 1;
-    const int x = 2 * ix2 + keo;
-    const int nx = 2 * p.nx2;
-    const int ieo = p.ieo;
-    const size_t strideMu = vh;          // links: ((ieo + 2*mu)*Vh + site)
-
-#define B200_HOP_DIR(MU, COORD, EXT, NBP, NBM)                                       \
-    {                                                                                \
-      R w[24], h[12], o[12], u[18];                                                  \
-      {                                                                              \
-        const R ph = (kPh || COORD != EXT - 1) ? R(1) : (R)p.bc[MU];                 \
-        const int nb = NBP;                                                          \
-        St::load(p.in, vh, LS, nb, s, w);                                            \
-        if (kDagHop) {                                                               \
-          _Pragma("unroll") for (int q = 0; q < 12; ++q) {                           \
-            R tmp = w[q]; w[q] = w[q + 12]; w[q + 12] = tmp; }                       \
-        }                                                                            \
-        project<R, MU, 1, !kPh>(w, h);                                               \
-        LinkLoad<LF>::load(p.links, (size_t)(ieo + 2 * MU) * strideMu + site, u);    \
-        su3_mult_half<R, false>(u, h, o);                                            \
-        reconstruct_acc<R, MU, 1, kPh>(acc, o, ph);                                  \
-      }                                                                              \
-      {                                                                              \
-        const R ph = (kPh || COORD != 0) ? R(1) : (R)p.bc[MU];                       \
-        const int nb = NBM;                                                          \
-        St::load(p.in, vh, LS, nb, s, w);                                            \
-        if (kDagHop) {                                                               \
-          _Pragma("unroll") for (int q = 0; q < 12; ++q) {                           \
-            R tmp = w[q]; w[q] = w[q + 12]; w[q + 12] = tmp; }                       \
-        }                                                                            \
-        project<R, MU, -1, !kPh>(w, h);                                              \
-        LinkLoad<LF>::load(p.links, (size_t)(1 - ieo + 2 * MU) * strideMu + nb, u);  \
-        su3_mult_half<R, true>(u, h, o);                                             \
-        reconstruct_acc<R, MU, -1, kPh>(acc, o, ph);                                 \
-      }                                                                              \
-    }
-
+    x = 2 * ix2 + keo;
     const int row = p.nx2 * iyzt;
-    B200_HOP_DIR(0, x, nx,
-                 row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo),
-                 row + ((ix2 - 1 + keo < 0) ? p.nx2 - 1 : ix2 - 1 + keo));
-    const int sy = p.nx2;
-    B200_HOP_DIR(1, y, p.ny,
-                 (y == p.ny - 1) ? site - (p.ny - 1) * sy : site + sy,
-                 (y == 0) ? site + (p.ny - 1) * sy : site - sy);
-    const int sz = p.nx2 * p.ny;
-    B200_HOP_DIR(2, z, p.nz,
-                 (z == p.nz - 1) ? site - (p.nz - 1) * sz : site + sz,
-                 (z == 0) ? site + (p.nz - 1) * sz : site - sz);
-    const int st = p.nx2 * p.ny * p.nz;
-    B200_HOP_DIR(3, t, p.nt,
-                 (t == p.nt - 1) ? site - (p.nt - 1) * st : site + st,
-                 (t == 0) ? site + (p.nt - 1) * st : site - st);
-#undef B200_HOP_DIR
+    nb[0] = row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo);
+    nb[1] = row + ((ix2 - 1 + keo < 0) ? p.nx2 - 1 : ix2 - 1 + keo);
+    const int sy = p.nx2, sz = p.nx2 * p.ny, st4 = p.nx2 * p.ny * p.nz;
+    nb[2] = (y == p.ny - 1) ? site - (p.ny - 1) * sy : site + sy;
+    nb[3] = (y == 0) ? site + (p.ny - 1) * sy : site - sy;
+    nb[4] = (z == p.nz - 1) ? site - (p.nz - 1) * sz : site + sz;
+    nb[5] = (z == 0) ? site + (p.nz - 1) * sz : site - sz;
+    nb[6] = (t == p.nt - 1) ? site - (p.nt - 1) * st4 : site + st4;
+    nb[7] = (t == 0) ? site + (p.nt - 1) * st4 : site - st4;
+  }
+  if constexpr (LSt::on) {
+    unsigned int* rec = reinterpret_cast<unsigned int*>(wbase + LSt::records * 144);
+    // record of direction d: forward U_mu(x) of this parity, backward
+    // U_mu(x-mu) of the other; past the last site, record 0 (never used)
+    if (g < G) {
+#pragma unroll
+      for (int d = 0; d < 8; ++d)
+        if (d % LS == s) {
+          const unsigned int pm = (unsigned int)(((d & 1) ? 1 - p.ieo : p.ieo) + (d & ~1));
+          rec[g * 8 + d] = active ? pm * (unsigned int)p.vh + (unsigned int)((d & 1) ? nb[d] : site) : 0u;
+        }
+    }
+    __syncwarp();
+    const uint32_t dst = smem_u32(wbase);
+    for (int i = lane; i < LSt::records * 9; i += 32) {
+      const int r = i / 9;
+      async_copy16(dst + i * 16, reinterpret_cast<const unsigned char*>(p.links) + (size_t)rec[r] * 144 + (i - 9 * r) * 16);
+    }
+  }
+  pdl_wait();
+  if (p.skip && *p.skip != 0.0) {
+    async_copy_wait();
+    return;
   }
 
-  hop_epilogue<LS, P, EPI, FK>(p, k, acc, tile_all + (size_t)warp * TileWarp<R, LS, G>::v, red_warp, tid, lane,
+  R acc[24];
+#pragma unroll
+  for (int i = 0; i < 24; ++i) acc[i] = 0;
+  const double2* lrec = reinterpret_cast<const double2*>(wbase) + (g < G ? g : 0) * 8 * 9;
+
+#define B200_HOP_HALF(D, MU, SIGN, EDGE)                                             \
+  {                                                                                  \
+    R w[24], h[12], o[12], u[18];                                                    \
+    if (active) St::load(p.in, vh, LS, nb[D], s, w);                                 \
+    if (LSt::on && D == 0) {                                                         \
+      async_copy_wait();                                                             \
+      __syncwarp();                                                                  \
+    }                                                                                \
+    if (active) {                                                                    \
+      if (kDagHop) {                                                                 \
+        _Pragma("unroll") for (int q = 0; q < 12; ++q) {                             \
+          R tmp = w[q]; w[q] = w[q + 12]; w[q + 12] = tmp; }                         \
+      }                                                                              \
+      project<R, MU, SIGN, !kPh>(w, h);                                              \
+      if constexpr (LSt::on) {                                                       \
+        hop_dir_rows_f64<MU, SIGN>(lrec + (D) * 9, reinterpret_cast<const double*>(h), \
+                                   reinterpret_cast<double*>(acc));                  \
+      } else {                                                                       \
+        const R ph = (kPh || !(EDGE)) ? R(1) : (R)p.bc[MU];                          \
+        LinkLoad<LF>::load(p.links, SIGN > 0 ? (size_t)(p.ieo + 2 * MU) * vh + site  \
+                                             : (size_t)(1 - p.ieo + 2 * MU) * vh + nb[D], u); \
+        su3_mult_half<R, (SIGN < 0)>(u, h, o);                                       \
+        reconstruct_acc<R, MU, SIGN, kPh>(acc, o, ph);                               \
+      }                                                                              \
+    }                                                                                \
+  }
+  B200_HOP_HALF(0, 0, 1, x == 2 * p.nx2 - 1)
+  B200_HOP_HALF(1, 0, -1, x == 0)
+  B200_HOP_HALF(2, 1, 1, y == p.ny - 1)
+  B200_HOP_HALF(3, 1, -1, y == 0)
+  B200_HOP_HALF(4, 2, 1, z == p.nz - 1)
+  B200_HOP_HALF(5, 2, -1, z == 0)
+  B200_HOP_HALF(6, 3, 1, t == p.nt - 1)
+  B200_HOP_HALF(7, 3, -1, t == 0)
+#undef B200_HOP_HALF
+
+  if (LSt::on) __syncwarp();     // the tile takes the links' place
+  hop_epilogue<LS, P, EPI, FK>(p, k, acc, reinterpret_cast<R*>(wbase), red_warp, tid, lane,
                                warp, g, s, site, active);
 }
 
@@ -719,8 +764,8 @@ __device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, 
   reconstruct_acc<R, MU, -1, kPh>(acc, o, (kPh || !firstm) ? R(1) : (R)p.bc[MU]);
 }
 
-template <int LS, int P, int LF, int EPI, int FK>
-__global__ void __launch_bounds__(128, 2)
+template <int LS, int P, int LF, int EPI, int FK, int MB>
+__global__ void __launch_bounds__(128, MB)
 dwf_hop_split_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
   pdl_launch_dependents();
   pdl_wait();
@@ -1602,10 +1647,9 @@ constexpr size_t hop_tma_smem_bytes() {
   return (size_t)4 * ((TmaGeom<LS, P, LF>::template warp_bytes<S>() + 127) / 128 * 128);
 }
 
-template <int LS, int P>
-constexpr size_t hop_smem_bytes() {
-  using R = typename Store<P>::R;
-  return sizeof(R) * (4 * TileWarp<R, LS, 32 / LS>::v);
+template <int LS, int P, int LF>
+constexpr size_t hop_direct_smem_bytes() {
+  return (size_t)4 * hop_direct_warp_bytes<LS, P, LF>();
 }
 
 }  // namespace b200

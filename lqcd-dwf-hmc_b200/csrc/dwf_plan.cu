@@ -220,6 +220,9 @@ int ensure_link_format(b200_dwf* op, int lf, cudaStream_t st) {
     if (cudaMalloc(&op->links[lf], link_bytes(lf, op->g.vh)) != cudaSuccess)
       return fail(B200_ENOMEM, "cudaMalloc for links failed");
     B200_CHECK_CUDA(launch_links_from_lex(lf, op->links[lf], op->u_lex, op->g, op->bc, st));
+    // the hops fetch links before they wait for earlier kernels (set_config
+    // waits for its conversions for the same reason)
+    B200_CHECK_CUDA(cudaStreamSynchronize(st));
   }
   return 0;
 }
@@ -273,11 +276,11 @@ SopParams sop_base(const b200_dwf* op) {
 // B200_AUTOTUNE=0 disables tuning (variant 0).  The first call of a
 // combination must not be inside a CUDA graph capture.
 typedef std::tuple<int, int, int, int, int> TuneKey;   // vh, ls, prec, epi, fk
-constexpr int kHopVariants = 11;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
+constexpr int kHopVariants = 12;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
                                   // higher occupancy, packed two-slice FP32x2 (direct, TMA),
                                   // 4-deep TMA, packed with all directions in flight, packed
                                   // half-storage with register prefetch, the four axes on
-                                  // four warps
+                                  // four warps (two register budgets)
 // Above this many sites every SM has several blocks of the other variants and
 // the split kernel's extra pass through shared memory only costs (FP64 D_eo
 // at 16^3x32, 65,536 sites: it is the slowest of the variants); its block
@@ -285,7 +288,7 @@ constexpr int kHopVariants = 11;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-st
 constexpr int kSplitMaxSites = 16384;
 
 bool variant_supported(int prec, int ls, int vh, int v) {
-  if (v == kHopSplit) return vh <= kSplitMaxSites;
+  if (v == kHopSplit || v == kHopSplit4) return vh <= kSplitMaxSites;
   if (v < 5) return true;
   if (v == 7 && prec == PREC_F64) return true;
   if (v == 9 && (prec == PREC_F64 || prec == PREC_F32)) return false;

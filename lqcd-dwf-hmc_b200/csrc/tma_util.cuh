@@ -107,6 +107,13 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
       : "memory");
 }
 
+// 16 bytes from global to shared memory without a register in between; waited
+// for by the issuing thread.
+__device__ __forceinline__ void async_copy16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Ask for `bytes` (multiple of 16, 16-byte aligned address) of global memory
 // to be brought into L2; completes nothing and waits for nothing.
 __device__ __forceinline__ void l2_prefetch(const void* src, uint32_t bytes) {

@@ -1,5 +1,5 @@
-"""The hop kernel that puts the four axes on four warps (chosen for small
-lattices): every mode and its dagger, every storage precision, against the CPU
+"""The hop kernels of small lattices, which put the four axes on four warps, and
+the direct ones: every mode and its dagger, every storage precision, against the CPU
 oracle, where its blocks are ragged (sites not a multiple of a warp's), where
 a warp has idle lanes (Ls 6, 12), on extents of 2 (one site is both
 neighbours) and with each boundary phase; and a solve, whose block sums come
@@ -24,11 +24,15 @@ CASES = [
 TOL = {0: 1e-13, 1: 5e-6, 2: 5e-3, 3: 4e-2}
 
 
+# 10, 11: the split kernel at its two register budgets; 0, 4: the direct kernel,
+# whose FP64 links a warp stages for all its sites (at Ls 4 more of them than
+# the epilogue's tile takes, at Ls 4 and 6 fewer lanes per site than directions)
+@pytest.mark.parametrize("variant", ["10", "11", "0", "4"])
 @pytest.mark.parametrize("ci", range(len(CASES)))
-def test_split_hop_against_oracle(ci, monkeypatch):
+def test_split_and_direct_hops_against_oracle(ci, variant, monkeypatch):
     import b200dwf
     from oracle.oracle import OracleDWF
-    monkeypatch.setenv("B200_HOP_VARIANT", "10")
+    monkeypatch.setenv("B200_HOP_VARIANT", variant)
     lat, ls, b, c, bc = CASES[ci]
     u = synth.gauge_field(lat, 60 + ci, "hot")
     w = synth.spinor_field(lat, ls, 70 + ci)
