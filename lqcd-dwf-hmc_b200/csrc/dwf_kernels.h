@@ -96,7 +96,8 @@ struct MsUpdParams {
   double* red;           // partials [kMaxShift][nblocks] of |p_i|^2
   int nblocks;
   Geom g;
-  void* const* win;      // windowed mode: device array [kMaxWin] of residual slots (else null)
+  void* const* win;      // windowed mode: device array [kMaxWin] of residual slots (else null);
+                         // r is the slot that this iteration's hop wrote
   void* p0s;             // windowed mode with x_0 deferred to the flush: p_0 at the window's
                          // start (else null; x_0 is then updated every iteration)
 };

@@ -1031,7 +1031,6 @@ static int cg_core(b200_dwf_t* op, int prec, void* x, const void* b, int maxiter
   const double start[4] = {0.0, 0.0, bnorm2, tol2};    // SC_DONE, SC_ITER, SC_BNORM, SC_TOL2
   B200_CHECK_CUDA(cudaMemcpyAsync(op->sc + SC_DONE, start, sizeof(start), cudaMemcpyHostToDevice, st));
   const double* done = op->sc + SC_DONE;
-
   auto iteration = [&](int it) -> int {
     HopParams p1 = hop_base(op, prec, 1, EPI_K1);
     p1.in = yp; p1.out1 = y1; p1.skip = done;
@@ -1214,10 +1213,10 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
   // start: 2 field passes less per iteration against 5 more per window)
   const int window = op->ms_window;
   void* p0s = nullptr;
+  std::vector<void*> wp(kMaxWin, nullptr);
   if (window > 0) {
     if (!op->ms_win_ptrs && cudaMalloc(&op->ms_win_ptrs, kMaxWin * sizeof(void*)) != cudaSuccess)
       return fail(B200_ENOMEM, "cudaMalloc for multishift window pointers failed");
-    std::vector<void*> wp(kMaxWin, nullptr);
     for (int l = 0; l < window; ++l)
       if (ms_pool_slot(op->ws->win, l, fbytes, &wp[l]))
         return fail(B200_ENOMEM, "cudaMalloc for multishift window slot %d failed", l);
@@ -1284,7 +1283,12 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
   // One iteration: the four fused DdagD hops, the scalar steps and the fused
   // update of every active shift.  Every kernel skips itself once S[MS_DONE]
   // is set, so iterations can be replayed past convergence as no-ops.
-  auto iteration = [&](cudaStream_t s) -> int {
+  // Iteration `it` of the solve: in windowed mode the residual that its last
+  // hop writes goes straight into window slot it mod m, and the one it reads is
+  // the previous iteration's slot, so no pass copies residuals.
+  auto iteration = [&](int it, cudaStream_t s) -> int {
+    void* r_in = window > 0 && it > 0 ? wp[(it - 1) % window] : r;
+    void* r_out = window > 0 ? wp[it % window] : r;
     int rc2;
     HopParams p1 = hop_base(op, prec, 1, EPI_K1);
     p1.in = y0; p1.out1 = y1; p1.skip = S + MS_DONE;
@@ -1299,16 +1303,16 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
     if ((rc2 = run_hop(op, prec, p3, s))) return rc2;
     // r += beta (DdagD p0 + sigma0 p0) = r + beta t2 + beta sigma0 p0 + beta K4N(hop)
     HopParams p4 = hop_base(op, prec, 0, EPI_K4N);
-    p4.in = t3; p4.out1 = r;
+    p4.in = t3; p4.out1 = r_out;
     p4.ce = 1.0; p4.ce_dev = S + MS_BETA;
-    p4.x1 = r; p4.c_x1 = 1.0;
+    p4.x1 = r_in; p4.c_x1 = 1.0;
     p4.x2 = t2; p4.c_x2 = 1.0; p4.c_x2_dev = S + MS_BETA;
     p4.x3 = p0; p4.c_x3 = sigma[0]; p4.c_x3_dev = S + MS_BETA;
     p4.red = op->red; p4.skip = S + MS_DONE;
     if ((rc2 = run_hop(op, prec, p4, s))) return rc2;
     B200_CHECK_CUDA(launch_ms_scalar(MSS_ALPHA, op->red, hop_partials(p4.variant, g.ls, g.vh), S, nshift, s));
     MsUpdParams mu;
-    mu.xs = op->ms_ptrs; mu.ps = op->ms_ptrs + kMaxShift; mu.r = r; mu.y0 = op->m5pre_id ? nullptr : y0;
+    mu.xs = op->ms_ptrs; mu.ps = op->ms_ptrs + kMaxShift; mu.r = r_out; mu.y0 = op->m5pre_id ? nullptr : y0;
     mu.st = S; mu.red = op->ms_red; mu.nblocks = nb_hop; mu.g = g;
     mu.win = window > 0 ? op->ms_win_ptrs : nullptr;
     mu.p0s = p0s;
@@ -1337,20 +1341,21 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
   double done = 0.0, iters = 0.0, rr = bnorm2;
   if (maxiter > 0) {
     // the first iteration runs on the caller's stream (it may autotune the
-    // four hop epilogues); the rest replay a captured CUDA graph of kBatch
-    // iterations on a private stream, checking the device's stop flag after
-    // each replay
-    if ((rc = iteration(st))) return rc;
+    // four hop epilogues); the rest replay a captured CUDA graph of `batch`
+    // iterations (whole windows, so that every replay meets the same slots) on
+    // a private stream, checking the device's stop flag after each replay
+    if ((rc = iteration(0, st))) return rc;
     if ((rc = read_state(st, &done, &iters, &rr))) return rc;
     if (done == 0.0) {
       constexpr int kBatch = 16;
+      const int batch = window > 0 ? window * ((kBatch + window - 1) / window) : kBatch;
       if (!op->gst && cudaStreamCreateWithFlags(&op->gst, cudaStreamNonBlocking) != cudaSuccess)
         return fail(B200_ECUDA, "cudaStreamCreate failed");
       cudaGraph_t graph = nullptr;
       cudaGraphExec_t exec = nullptr;
       B200_CHECK_CUDA(cudaStreamBeginCapture(op->gst, cudaStreamCaptureModeThreadLocal));
       int rc_cap = 0;
-      for (int b2 = 0; b2 < kBatch && !rc_cap; ++b2) rc_cap = iteration(op->gst);
+      for (int b2 = 0; b2 < batch && !rc_cap; ++b2) rc_cap = iteration(1 + b2, op->gst);
       const cudaError_t ec = cudaStreamEndCapture(op->gst, &graph);
       if (rc_cap) { if (graph) cudaGraphDestroy(graph); return rc_cap; }
       B200_CHECK_CUDA(ec);

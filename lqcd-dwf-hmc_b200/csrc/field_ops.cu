@@ -380,11 +380,7 @@ ms_update_kernel(MsUpdParams p, const __grid_constant__ ChainCoef<typename Store
     }
   }
   block_reduce_store(nrm, p.red);
-  if (p.win) {
-    // windowed mode: keep this iteration's residual; the shifts follow later
-    if (active) St::store(p.win[(int)p.st[MS_WIN]], vh, LS, site, s, rv);
-    return;
-  }
+  if (p.win) return;   // windowed mode: r is a window slot already; the shifts follow later
   for (int ish = 1; ish < nact; ++ish) {
     __syncthreads();
     const R bs = (R)p.st[MS_N + MSA_BETAS * kMaxShift + ish];
