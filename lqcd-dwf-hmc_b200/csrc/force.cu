@@ -24,6 +24,19 @@ namespace b200 {
 // doubles so that the warp's stores miss no bank.
 constexpr int kRow = 19;
 
+// Where a site's results go, worked out once by the site's first lane: formed
+// for every output and direction again, the divisions were more than a third
+// of the kernel's 92 M warp instructions at 16^3x32 Ls=16 (29 M of them FP64).
+// Bound by latency at 8 warps an SM (226 registers): both parities at 24^3x48
+// Ls=16 2.49 -> 2.14 ms.  Two warps a site set, one term each, at 12 warps an
+// SM: 2.34 ms, the doubled reduction rows cost more than the warps gain; the
+// parities side by side in one launch: no difference.
+struct ForceSite {
+  long long lex;      // lexical site index
+  int edge;           // bit mu: x -> x+mu crosses the boundary
+  int live;
+};
+
 template <int LS, bool T1, bool T2>
 __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
   using St = Store<PREC_F64>;
@@ -31,6 +44,7 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
   constexpr int G = 32 / LS;
   constexpr int WARPS = 4;
   extern __shared__ unsigned char smem_raw[];
+  __shared__ ForceSite where[WARPS][G];
   R* tile = reinterpret_cast<R*>(smem_raw) + (size_t)(threadIdx.x >> 5) * G * LS * kRow;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane / LS;
@@ -50,13 +64,20 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
     keo = (p.ieo + y + z + t) & 1;
     x = 2 * ix2 + keo;
   }
+  if (g < G && s == 0) {
+    ForceSite w;
+    w.lex = x + (long long)(2 * p.nx2) * iyzt;
+    w.edge = (x == 2 * p.nx2 - 1 ? 1 : 0) | (y == p.ny - 1 ? 2 : 0) | (z == p.nz - 1 ? 4 : 0) | (t == p.nt - 1 ? 8 : 0);
+    w.live = active;
+    where[warp][g] = w;
+  }
   R z1[24], z2[24];
   if (active) {
     if (T1) St::load(p.z1, vh, LS, site, s, z1);
     if (T2) St::load(p.z2, vh, LS, site, s, z2);
   }
 
-#define B200_FORCE_MU(MU, EXT, NBP)                                                   \
+#define B200_FORCE_MU(MU, NBP)                                                        \
   {                                                                                   \
     R f[18];                                                                          \
     _Pragma("unroll") for (int i = 0; i < 18; ++i) f[i] = 0;                          \
@@ -99,30 +120,24 @@ __global__ void __launch_bounds__(128) force_kernel(ForceParams p) {
     __syncwarp();                                                                     \
     for (int o = lane; o < 18 * G; o += 32) {                                         \
       const int gg = o / 18, i = o - 18 * gg;                                         \
-      const int st = (blockIdx.x * WARPS + warp) * G + gg;                            \
-      if (st < p.vh) {                                                                \
+      const ForceSite w = where[warp][gg];                                            \
+      if (w.live) {                                                                   \
         R sum = 0;                                                                    \
-        for (int q = 0; q < LS; ++q) sum += tile[(gg * LS + q) * kRow + i];           \
-        const int sx2 = st % p.nx2, syzt = st / p.nx2;                                \
-        const int sy = syzt % p.ny, sz = (syzt / p.ny) % p.nz, stt = syzt / (p.ny * p.nz); \
-        const int sxx = 2 * sx2 + ((p.ieo + sy + sz + stt) & 1);                      \
-        const int coord = MU == 0 ? sxx : MU == 1 ? sy : MU == 2 ? sz : stt;          \
-        const size_t lex = sxx + (size_t)(2 * p.nx2) *                                \
-                           (sy + (size_t)p.ny * (sz + (size_t)p.nz * stt));           \
-        double* dst = p.force + 18 * (lex + (size_t)2 * vh * MU) + i;                 \
-        const R cf = coord == (EXT) - 1 ? p.coef * p.bc[MU] : p.coef;                 \
+        _Pragma("unroll") for (int q = 0; q < LS; ++q) sum += tile[(gg * LS + q) * kRow + i]; \
+        double* dst = p.force + 18 * ((size_t)w.lex + (size_t)2 * vh * MU) + i;       \
+        const R cf = (w.edge >> MU) & 1 ? p.coef * p.bc[MU] : p.coef;                 \
         *dst = (p.beta != 0.0 ? p.beta * (*dst) : 0.0) + cf * sum;                    \
       }                                                                               \
     }                                                                                 \
   }
 
   const int row = p.nx2 * iyzt;
-  B200_FORCE_MU(0, 2 * p.nx2, row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo))
-  B200_FORCE_MU(1, p.ny, (y == p.ny - 1) ? site - (p.ny - 1) * p.nx2 : site + p.nx2)
+  B200_FORCE_MU(0, row + ((ix2 + keo == p.nx2) ? 0 : ix2 + keo))
+  B200_FORCE_MU(1, (y == p.ny - 1) ? site - (p.ny - 1) * p.nx2 : site + p.nx2)
   const int sz_ = p.nx2 * p.ny;
-  B200_FORCE_MU(2, p.nz, (z == p.nz - 1) ? site - (p.nz - 1) * sz_ : site + sz_)
+  B200_FORCE_MU(2, (z == p.nz - 1) ? site - (p.nz - 1) * sz_ : site + sz_)
   const int st_ = p.nx2 * p.ny * p.nz;
-  B200_FORCE_MU(3, p.nt, (t == p.nt - 1) ? site - (p.nt - 1) * st_ : site + st_)
+  B200_FORCE_MU(3, (t == p.nt - 1) ? site - (p.nt - 1) * st_ : site + st_)
 #undef B200_FORCE_MU
 }
 
