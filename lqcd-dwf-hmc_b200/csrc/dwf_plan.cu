@@ -281,11 +281,12 @@ constexpr int kHopVariants = 12;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-st
                                   // 4-deep TMA, packed with all directions in flight, packed
                                   // half-storage with register prefetch, the four axes on
                                   // four warps (two register budgets)
-// Above this many sites every SM has several blocks of the other variants and
-// the split kernel's extra pass through shared memory only costs (FP64 D_eo
-// at 16^3x32, 65,536 sites: it is the slowest of the variants); its block
-// partials fit the plan's buffer up to here.
-constexpr int kSplitMaxSites = 16384;
+// The split kernel's range: at 256 sites (4^3x8, Ls 8) it takes DdagD from 50.7
+// to 40.1 us; at 2,048 it is level with the direct kernels (FP64 D_eo^+ Ls 8:
+// 8.5 against 8.6 us, Ls 12: 9.1 against 8.6), at 4,096 every SM has several
+// blocks and it is the slower one (Ls 12: 14.7 against 9.7 us, at 13,824 sites
+// 44.6 against 28.4).  Its block partials fit the plan's buffer up to here.
+constexpr int kSplitMaxSites = 2048;
 
 bool variant_supported(int prec, int ls, int vh, int v) {
   if (v == kHopSplit || v == kHopSplit4) return vh <= kSplitMaxSites;
@@ -328,7 +329,11 @@ int tune_hop(b200_dwf* op, int prec, const HopParams& p0, cudaStream_t st, int* 
   // variants are timed in turn, round after round, and each keeps its
   // fastest round: a clock change then touches every variant alike instead
   // of whichever was timed during it.
-  constexpr int kRounds = 3, kReps = 2;
+  // Launches of a few microseconds are timed more at a time: between two of
+  // them the spread of the events alone is larger than what tells the variants
+  // apart (the 8^4 CG took 6.9 or 7.5 ms with the picks of two launches).
+  constexpr int kRounds = 3;
+  const int kReps = op->g.vh <= 16384 ? 8 : 2;
   int vs[kHopVariants];
   float t[kHopVariants];
   int nv = 0;
