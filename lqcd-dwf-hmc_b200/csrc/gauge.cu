@@ -399,12 +399,15 @@ int b200_gauge_force_rect(const int lattice[4], double beta, double c_plaq, doub
   cudaStream_t st = (cudaStream_t)stream;
   const dim3 grid((unsigned)((g.vol + 127) / 128), 4);
   // The planar copy costs one pass over the links and makes the 66 link loads
-  // of a thread whole lines; without room for it the links are read where
-  // they are (same arithmetic, 16^3x32: 3.5x slower).
+  // of a thread whole lines.  Without room for it, and in a stream capture
+  // (whose graph would own the copy and could be instantiated only once), the
+  // links are read where they are, with the same arithmetic.
   double2* planar = nullptr;
-  cudaMemPool_t pool = scratch_pool();
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+  cudaMemPool_t pool = capture == cudaStreamCaptureStatusNone ? scratch_pool() : nullptr;
   if (!pool || cudaMallocFromPoolAsync((void**)&planar, 4 * g.vol * 9 * sizeof(double2), pool, st) != cudaSuccess) {
-    cudaGetLastError();
+    if (pool) cudaGetLastError();
     gauge_force_kernel<<<grid, 128, 0, st>>>(LexField{u, (unsigned)g.vol}, force, g, beta, c_plaq, c_rect);
     G_CHECK(cudaGetLastError());
     return 0;

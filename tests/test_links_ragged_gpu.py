@@ -131,3 +131,25 @@ def test_links_axpby_alignment(lat, off):
     assert torch.equal(y, 2.0 * x)
     b200dwf.check(b200dwf.lib().b200_momentum_update(L, 0.5, p(x), p(y), None))
     assert torch.equal(y, 2.5 * x)
+
+
+def test_gauge_force_under_capture():
+    """A captured call, which reads the links where they are, replays to the
+    same force as a direct one."""
+    import torch
+    import b200dwf
+    lat = [6, 4, 2, 6]
+    u = torch.from_numpy(synth.gauge_field(lat, 9, "hot")).cuda()
+    L = (ctypes.c_int * 4)(*lat)
+    a, b = torch.zeros_like(u), torch.zeros_like(u)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    call = b200dwf.lib().b200_gauge_force_rect
+    b200dwf.check(call(L, 2.13, 3.648, -0.331, p(a), p(u), None))
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        b200dwf.check(call(L, 2.13, 3.648, -0.331, p(b), p(u), st))
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.max(torch.abs(a - b)).item() < 1e-13
