@@ -316,7 +316,9 @@ int b200_smear_destroy(b200_smear_t *sm);
 /* set_config + smear: u = thin links (host if on_device == 0, else device). */
 int b200_smear_set_config(b200_smear_t *sm, const double *u, int on_device, void *stream);
 /* Device pointer of smearing level `level` (0 = thin links, nsmear = fully
- * smeared); NULL if out of range or no config was set. */
+ * smeared); NULL if out of range or no config was set, or if a level below
+ * the top, whose copy in this layout is made on the first request, does not
+ * fit.  A pointer handed out stays that level's through later set_config. */
 const double *b200_smear_config(b200_smear_t *sm, int level);
 /* Copy of level `level` to host memory (18*4*Nvol doubles). */
 int b200_smear_get_config(b200_smear_t *sm, int level, double *host_out, void *stream);
