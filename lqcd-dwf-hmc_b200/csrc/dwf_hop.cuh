@@ -1059,98 +1059,68 @@ __device__ __forceinline__ void pair_fetch(const HopParams& p, int nb, size_t li
   r.l2 = __ldg(lp + 2);
 }
 
-template <int P>
+// the stored components of one slice in FP32, spins swapped for the
+// gamma5-sandwiched dagger hop
+template <int P, bool kDagHop>
 __device__ __forceinline__ void pair_decode(const uint4 (&c)[3], float* v) {
   using HO = HalfOps<typename Store<P>::Half>;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float2 a = HO::to2(c[k].x), b = HO::to2(c[k].y), d = HO::to2(c[k].z), e = HO::to2(c[k].w);
-    v[8 * k + 0] = a.x; v[8 * k + 1] = a.y; v[8 * k + 2] = b.x; v[8 * k + 3] = b.y;
-    v[8 * k + 4] = d.x; v[8 * k + 5] = d.y; v[8 * k + 6] = e.x; v[8 * k + 7] = e.y;
+    const unsigned int w[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = HO::to2(w[i]);
+      const int q = kDagHop ? (8 * k + 2 * i + 12) % 24 : 8 * k + 2 * i;
+      v[q] = a.x;
+      v[q + 1] = a.y;
+    }
   }
 }
 
-// The Dirac-basis projection (1 - sign*gamma_mu) of project(), applied to the
-// stored (re, im) half-precision pairs before any conversion to FP32: each
-// projected colour is one paired multiply-add, h = w_a + f * w_b or
-// w_a + f * swap(w_b) with f = (+-1, +-1), so a slice converts 6 pairs instead
-// of 12 and issues 6 paired operations instead of 12 FP32 adds.  The rounding
-// this adds is that of the storage format itself.  w[c + 3*spin],
-// h[c + 3*a]; t projection without its factor 2 (folded into the links).
-template <typename H2> struct Half2Ops;
-template <> struct Half2Ops<__half2> {
-  __device__ static __half2 k(float a, float b) { return __floats2half2_rn(a, b); }
-  __device__ static float2 f2(__half2 h) { return __half22float2(h); }
-};
-template <> struct Half2Ops<__nv_bfloat162> {
-  __device__ static __nv_bfloat162 k(float a, float b) { return __floats2bfloat162_rn(a, b); }
-  __device__ static float2 f2(__nv_bfloat162 h) { return __bfloat1622float2(h); }
-};
-
-template <typename H2, int MU, int SIGN>
-__device__ __forceinline__ void project_half2(const H2* w, H2* h) {
-  using O = Half2Ops<H2>;
-  constexpr float S = SIGN > 0 ? 1.f : -1.f;
+// project() of two slices at once, w and h as (slice s0, slice s1) pairs: each
+// sum is one packed multiply-add by +-1, which rounds as the FP32 sum does, so
+// the results are those of dwf_hop_pair_kernel bit for bit and the autotuner
+// chooses among kernels of one arithmetic.  (Projecting the stored pairs in
+// half precision took 1557 us for DdagD at 24^3x48 Ls=16 f16 against 1589 us
+// this way, but made the rounding of the operator a matter of which kernel was
+// timed the faster: error against 64 bits 4.0e-4 then, 3.7e-4 now.)  t
+// projection without its factor 2 (folded into the links).
+template <int MU, int SIGN>
+__device__ __forceinline__ void project2(const float2* w, float2* h) {
+  const float2 pos = f2(SIGN > 0 ? 1.f : -1.f), neg = f2(SIGN > 0 ? -1.f : 1.f);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const H2 w0 = w[c], w1 = w[c + 3], w2 = w[c + 6], w3 = w[c + 9];
-    H2 h0, h1;
-    if (MU == 0) {        // h0 = w0 -+ i w3, h1 = w1 -+ i w2 (as project)
-      h0 = __hfma2(__lowhigh2highlow(w3), O::k(-S, S), w0);
-      h1 = __hfma2(__lowhigh2highlow(w2), O::k(-S, S), w1);
+    const float2* w0 = w + 2 * c;
+    const float2* w1 = w + 2 * (c + 3);
+    const float2* w2 = w + 2 * (c + 6);
+    const float2* w3 = w + 2 * (c + 9);
+    float2* h0 = h + 2 * c;
+    float2* h1 = h + 6 + 2 * c;
+    if (MU == 0) {        // h0 = w0 +- i w3, h1 = w1 +- i w2
+      h0[0] = __ffma2_rn(neg, w3[1], w0[0]); h0[1] = __ffma2_rn(pos, w3[0], w0[1]);
+      h1[0] = __ffma2_rn(neg, w2[1], w1[0]); h1[1] = __ffma2_rn(pos, w2[0], w1[1]);
     } else if (MU == 1) { // h0 = w0 +- w3, h1 = w1 -+ w2
-      h0 = __hfma2(w3, O::k(S, S), w0);
-      h1 = __hfma2(w2, O::k(-S, -S), w1);
-    } else if (MU == 2) { // h0 = w0 -+ i w2, h1 = w1 +- i w3
-      h0 = __hfma2(__lowhigh2highlow(w2), O::k(-S, S), w0);
-      h1 = __hfma2(__lowhigh2highlow(w3), O::k(S, -S), w1);
+      h0[0] = __ffma2_rn(pos, w3[0], w0[0]); h0[1] = __ffma2_rn(pos, w3[1], w0[1]);
+      h1[0] = __ffma2_rn(neg, w2[0], w1[0]); h1[1] = __ffma2_rn(neg, w2[1], w1[1]);
+    } else if (MU == 2) { // h0 = w0 +- i w2, h1 = w1 -+ i w3
+      h0[0] = __ffma2_rn(neg, w2[1], w0[0]); h0[1] = __ffma2_rn(pos, w2[0], w0[1]);
+      h1[0] = __ffma2_rn(pos, w3[1], w1[0]); h1[1] = __ffma2_rn(neg, w3[0], w1[1]);
     } else {              // (1 - g4) keeps the lower spins, (1 + g4) the upper
-      h0 = SIGN > 0 ? w2 : w0;
-      h1 = SIGN > 0 ? w3 : w1;
+      h0[0] = SIGN > 0 ? w2[0] : w0[0]; h0[1] = SIGN > 0 ? w2[1] : w0[1];
+      h1[0] = SIGN > 0 ? w3[0] : w1[0]; h1[1] = SIGN > 0 ? w3[1] : w1[1];
     }
-    h[c] = h0;
-    h[c + 3] = h1;
-  }
-}
-
-template <int P> struct Half2Of;
-template <> struct Half2Of<PREC_F16> { using T = __half2; };
-template <> struct Half2Of<PREC_BF16> { using T = __nv_bfloat162; };
-
-// the 12 stored pairs of one slice (three 16-byte chunks), spins swapped for
-// the gamma5-sandwiched dagger hop
-template <int P, bool kDagHop>
-__device__ __forceinline__ void pair_unpack(const uint4 (&c)[3], typename Half2Of<P>::T* w) {
-  using H2 = typename Half2Of<P>::T;
-  unsigned int u[12];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    u[4 * k] = c[k].x; u[4 * k + 1] = c[k].y; u[4 * k + 2] = c[k].z; u[4 * k + 3] = c[k].w;
-  }
-#pragma unroll
-  for (int q = 0; q < 12; ++q) {
-    const unsigned int v = kDagHop ? u[(q + 6) % 12] : u[q];
-    w[q] = *reinterpret_cast<const H2*>(&v);
   }
 }
 
 template <int P, int MU, int SIGN, bool kDagHop>
 __device__ __forceinline__ void pair_compute(const PairRaw<P>& r, float ph, float2* acc) {
-  using H2 = typename Half2Of<P>::T;
-  using O = Half2Ops<H2>;
-  float u[18];
-  H2 w0[12], w1[12], p0[6], p1[6];
-  pair_unpack<P, kDagHop>(r.c0, w0);
-  pair_unpack<P, kDagHop>(r.c1, w1);
-  project_half2<H2, MU, SIGN>(w0, p0);
-  project_half2<H2, MU, SIGN>(w1, p1);
-  float2 h[12], o[12];
+  float u[18], w0[24], w1[24];
+  pair_decode<P, kDagHop>(r.c0, w0);
+  pair_decode<P, kDagHop>(r.c1, w1);
+  float2 w[24], h[12], o[12];
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    const float2 a = O::f2(p0[q]), b = O::f2(p1[q]);
-    h[2 * q] = make_float2(a.x, b.x);
-    h[2 * q + 1] = make_float2(a.y, b.y);
-  }
+  for (int q = 0; q < 24; ++q) w[q] = make_float2(w0[q], w1[q]);
+  project2<MU, SIGN>(w, h);
   LinkLoad<LINK_F16_18>::decode(r.l0, r.l1, r.l2, u);
   su3_mult_half2<(SIGN < 0)>(u, h, o);
   reconstruct_acc2<MU, SIGN>(acc, o, make_float2(r.sc0 * ph, r.sc1 * ph));
