@@ -313,7 +313,9 @@ int b200_dwf_force_acc(b200_dwf_t *op, const char *mode, double *force, const vo
 typedef struct b200_smear b200_smear_t;
 int b200_smear_create(b200_smear_t **sm, const int lattice[4], double rho, int nsmear);
 int b200_smear_destroy(b200_smear_t *sm);
-/* set_config + smear: u = thin links (host if on_device == 0, else device). */
+/* set_config + smear: u = thin links (host if on_device == 0, else device: any
+ * array of doubles; one that is not on a 16-byte boundary or not memory of the
+ * current device is copied first). */
 int b200_smear_set_config(b200_smear_t *sm, const double *u, int on_device, void *stream);
 /* Device pointer of smearing level `level` (0 = thin links, nsmear = fully
  * smeared); NULL if out of range or no config was set, or if a level below

@@ -14,6 +14,7 @@
 // ri + 2*(col + 3*row) + 18*(site + Nvol*mu).
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 #include <vector>
 
@@ -438,6 +439,21 @@ static PlanarField planar_level(const b200_smear* sm, int level) {
   return PlanarField{sm->planar + (size_t)level * 36 * sm->g.vol, (unsigned)sm->g.vol};
 }
 
+// The planar copy reads the caller's links 16 bytes at a time and from this
+// device.  What it cannot read so (a view at an odd number of doubles, memory
+// of another device, page-locked host memory) is copied first, as host links
+// are.
+static bool readable_in_place(const double* u) {
+  if (reinterpret_cast<uintptr_t>(u) & 15u) return false;
+  int dev = 0;
+  cudaPointerAttributes a;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, u) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 static unsigned link_grid(const b200_smear* sm) { return (unsigned)((sm->g.vol + 31) / 32); }
 
 int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void* stream) {
@@ -447,8 +463,8 @@ int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void
   std::lock_guard<std::mutex> lock(sm->mu);
   double* top = sm->lex[sm->nsmear];
   const double* thin = u;
-  if (sm->nsmear == 0 || !on_device) {
-    // host links pass through the top level's buffer, which the last level
+  if (sm->nsmear == 0 || !on_device || !readable_in_place(u)) {
+    // these links pass through the top level's buffer, which the last level
     // overwrites once the planar copy has been made
     B200_SMEAR_CHECK(cudaMemcpyAsync(top, u, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
     thin = top;

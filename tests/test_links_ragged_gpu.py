@@ -133,6 +133,23 @@ def test_links_axpby_alignment(lat, off):
     assert torch.equal(y, 2.5 * x)
 
 
+@pytest.mark.parametrize("lat", LATS[:2])
+@pytest.mark.parametrize("off", [0, 1])
+def test_stout_set_config_alignment(lat, off):
+    """Device links on an 8-byte boundary that is not a 16-byte one smear to the
+    same levels as host links."""
+    import torch
+    import b200dwf
+    u = synth.gauge_field(lat, 3, "near", eps=0.3)
+    d = torch.empty(u.size + 1, dtype=torch.float64, device="cuda")[off:off + u.size]
+    d.copy_(torch.from_numpy(u))
+    a, b = b200dwf.StoutSmear(lat, 0.1, 2), b200dwf.StoutSmear(lat, 0.1, 2)
+    a.set_config(u)
+    b200dwf.check(b200dwf.lib().b200_smear_set_config(b.handle, ctypes.c_void_p(d.data_ptr()), 1, None))
+    for level in range(3):
+        assert np.array_equal(a.config(level), b.config(level)), level
+
+
 def test_gauge_force_under_capture():
     """A captured call, which reads the links where they are, replays to the
     same force as a direct one."""

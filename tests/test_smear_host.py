@@ -1,0 +1,29 @@
+"""Host code of the smearing plan on the fake CUDA runtime: which links
+set_config reads in place and which it copies first."""
+import pytest
+
+from fake_cuda import run
+
+
+@pytest.mark.parametrize("name,offset,kind,device,copied", [
+    ("device memory on a 16-byte boundary", 0, "DEVICE", 0, False),
+    ("device memory on an 8-byte boundary", 1, "DEVICE", 0, True),
+    ("memory of another device", 0, "DEVICE", 1, True),
+    ("page-locked host memory", 0, "HOST", 0, True),
+])
+def test_set_config_copies_what_its_kernel_cannot_read(tmp_path, name, offset, kind, device, copied):
+    run(tmp_path, """
+    sm = b200dwf.StoutSmear([4, 4, 4, 4], 0.1, 2)
+    u, p = array(nlink, %d)
+    fake.fake_pointer(p, %s, %d)
+    log()
+    b200dwf.check(lib.b200_smear_set_config(sm.handle, p, 1, None))
+    lines = log()
+    copies = [l for l in lines if l.startswith("memcpy") and hex(p.value) in l]
+    launches = [i for i, l in enumerate(lines) if l.startswith("launch")]
+    assert len(copies) == %d, lines
+    # the planar copy and two levels, after the links have been copied
+    assert len(launches) == 3, lines
+    if copies:
+        assert lines.index(copies[0]) < launches[0], lines
+    """ % (offset, kind, device, int(copied)))
