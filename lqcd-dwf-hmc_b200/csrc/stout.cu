@@ -374,6 +374,7 @@ struct b200_smear {
   double2* itheta = nullptr;
   double2* sig = nullptr;
   std::mutex mu;                   // guards the lexical copies made on request
+  int device = 0;                  // the device that the levels are on
   bool have_config = false;
 };
 
@@ -408,6 +409,7 @@ int b200_smear_create(b200_smear_t** out, const int lattice[4], double rho, int 
   sm->rho = rho;
   sm->nsmear = nsmear;
   sm->lex.assign(nsmear + 1, nullptr);
+  cudaGetDevice(&sm->device);
   const size_t n = nreal_cfg(sm) / 2;      // double2 of one field
   const size_t fields = nsmear > 0 ? nsmear + 3 : 1;
   if (sm->g.vol > 0x7fffffffu || cudaMalloc(&sm->block, fields * n * sizeof(double2)) != cudaSuccess) {
@@ -489,10 +491,14 @@ int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void
   return 0;
 }
 
-// A lexical copy of a level below the top, made on the first request: on a
-// stream of its own, so that a capture or work in progress on the caller's
-// streams is not touched (the levels are complete when set_config returns).
+// A lexical copy of a level below the top, made on the first request: on the
+// plan's device, whichever the calling thread has current, and on a stream of
+// its own, so that a capture or work in progress on the caller's streams is
+// not touched (the levels are complete when set_config returns).
 static int make_lex(b200_smear* sm, int level) {
+  int current = sm->device;
+  cudaGetDevice(&current);
+  if (current != sm->device) B200_SMEAR_CHECK(cudaSetDevice(sm->device));
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
   double* buf = nullptr;
@@ -505,9 +511,10 @@ static int make_lex(b200_smear* sm, int level) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
   if (st) cudaStreamDestroy(st);
+  if (e != cudaSuccess) cudaFree(buf);
   cudaThreadExchangeStreamCaptureMode(&mode);
+  if (current != sm->device) cudaSetDevice(current);
   if (e != cudaSuccess) {
-    cudaFree(buf);
     set_last_error(e == cudaErrorMemoryAllocation ? B200_ENOMEM : B200_ECUDA, "smear_config: %s", cudaGetErrorString(e));
     return B200_ECUDA;
   }

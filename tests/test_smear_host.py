@@ -27,3 +27,24 @@ def test_set_config_copies_what_its_kernel_cannot_read(tmp_path, name, offset, k
     if copies:
         assert lines.index(copies[0]) < launches[0], lines
     """ % (offset, kind, device, int(copied)))
+
+
+def test_level_copy_is_made_on_the_plans_device(tmp_path):
+    """A level's lexical copy, made on the first request, is on the device of
+    the plan whichever device the calling thread has current."""
+    run(tmp_path, """
+    sm = b200dwf.StoutSmear([4, 4, 4, 4], 0.1, 2)
+    u, p = array(nlink)
+    b200dwf.check(lib.b200_smear_set_config(sm.handle, p, 0, None))
+    fake.fake_device(1)
+    log()
+    assert lib.b200_smear_config(sm.handle, 0)
+    lines = log()
+    assert any(l.startswith("malloc") for l in lines) and any(l.startswith("launch") for l in lines), lines
+    for l in lines:
+        if "device" in l:
+            assert l.endswith("device 0"), lines
+    d = ctypes.c_int(-1)
+    fake.cudaGetDevice(ctypes.byref(d))
+    assert d.value == 1
+    """)
