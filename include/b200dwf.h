@@ -335,9 +335,15 @@ int b200_force_mult_generator(const int lattice[4], double *force, const double 
  * Device arrays in the lexical Field_G(Nvol, 4) layout (18 reals per link),
  * FP64.  Iwasaki / rectangle gauge action with beta, c_plaq, c_rect.
  * Force_G_Rectangle::force_core (src/lib/Force/Gauge/force_G_Rectangle.cpp:
- * 84-220): force = -(beta/3) TA(U_mu sum of staples^+), overwritten. */
+ * 84-220): force = -(beta/3) TA(U_mu sum of staples^+), overwritten.  The call
+ * uses scratch of the links' size, at most 2 GiB of which stays with the
+ * library between calls (b200_scratch_release; destroying a plan gives it back
+ * as well). */
 int b200_gauge_force_rect(const int lattice[4], double beta, double c_plaq, double c_rect,
                           double *force, const double *u, void *stream);
+/* Gives the scratch kept between calls back to the device: now, or, where work
+ * that uses it is still in flight, at the next synchronisation after it. */
+int b200_scratch_release(void);
 /* Action_G_Rectangle::calcH (src/lib/Action/Gauge/action_G_Rectangle.cpp:97-200);
  * synchronous. */
 int b200_gauge_action_rect(const int lattice[4], double beta, double c_plaq, double c_rect,

@@ -379,7 +379,23 @@ class DomainWall:
         return n.value, nf.value, d.value, rc
 
 
-class GaugeRect:
+class ScratchUser:
+    """Base of the objects whose calls use the scratch that the library keeps
+    between gauge forces; the last of them to go gives it back."""
+
+    _users = 0
+
+    def __new__(cls, *args, **kw):
+        ScratchUser._users += 1
+        return super().__new__(cls)
+
+    def __del__(self):
+        ScratchUser._users -= 1
+        if ScratchUser._users == 0 and _lib is not None:
+            _lib.b200_scratch_release()
+
+
+class GaugeRect(ScratchUser):
     """Iwasaki / rectangle gauge action (Force_G_Rectangle, Action_G_Rectangle)
     and the HMC link/momentum updates (Integrator_UpdateU/UpdateP,
     HMC_General::calcH_P) on device copies of lexical Field_G arrays."""

@@ -24,7 +24,7 @@ import time
 
 import numpy as np
 
-from . import check, lib
+from . import ScratchUser, check, lib
 
 
 def _p(t):
@@ -125,7 +125,7 @@ class Rational:
                 check(L.b200_dwf_force_acc(self.op.handle, b"DdagD", _p(out), x.ptr, None, bi, None))
 
 
-class GaugeMD:
+class GaugeMD(ScratchUser):
     """Leapfrog MD of the Iwasaki gauge action plus optional fermion actions."""
 
     def __init__(self, lattice, beta, c_plaq=3.648, c_rect=-0.331, nprec=8, fermions=()):

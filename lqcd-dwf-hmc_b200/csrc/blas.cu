@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 #include "dwf_kernels.h"
 
 namespace b200 {
@@ -128,7 +129,7 @@ int scratch(double** out, int* dev_out) {
   }
   *dev_out = dev;
   std::lock_guard<std::mutex> lk(g_mu);
-  if (!g_scratch[dev] && cudaMalloc(&g_scratch[dev], (2 * kBlocks + 2) * sizeof(double)) != cudaSuccess) {
+  if (!g_scratch[dev] && b200::device_malloc(&g_scratch[dev], (2 * kBlocks + 2) * sizeof(double)) != cudaSuccess) {
     g_scratch[dev] = nullptr;
     b200::set_last_error(B200_ENOMEM, "blas: cudaMalloc of the reduction scratch failed");
     return B200_ENOMEM;

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 #include "dwf_hop.cuh"
 #include "dwf_kernels.h"
 #include "learned.h"
@@ -144,7 +145,7 @@ static void workspace_release(Workspace* ws) {
 static int ms_pool_slot(std::vector<void*>& v, size_t i, size_t bytes, void** out) {
   std::lock_guard<std::mutex> lock(g_ws_mu);
   if (v.size() <= i) v.resize(i + 1, nullptr);
-  if (!v[i] && cudaMalloc(&v[i], bytes) != cudaSuccess) { v[i] = nullptr; return 1; }
+  if (!v[i] && device_malloc(&v[i], bytes) != cudaSuccess) { v[i] = nullptr; return 1; }
   *out = v[i];
   return 0;
 }
@@ -200,7 +201,7 @@ int ensure_work(b200_dwf* op, int prec, int i) {
   std::lock_guard<std::mutex> lock(g_ws_mu);
   if (!op->work[i][prec]) {
     const size_t bytes = field_bytes(prec, op->g.vh, op->g.ls);
-    if (cudaMalloc(&op->work[i][prec], bytes) != cudaSuccess) {
+    if (device_malloc(&op->work[i][prec], bytes) != cudaSuccess) {
       op->work[i][prec] = nullptr;
       return fail(B200_ENOMEM, "cudaMalloc of %zu bytes for a work field failed", bytes);
     }
@@ -217,7 +218,7 @@ int link_format_for(int prec) {
 int ensure_link_format(b200_dwf* op, int lf, cudaStream_t st) {
   if (!op->have_links) return fail(B200_EINVAL, "set_config has not been called on this operator");
   if (!op->links[lf]) {
-    if (cudaMalloc(&op->links[lf], link_bytes(lf, op->g.vh)) != cudaSuccess)
+    if (device_malloc(&op->links[lf], link_bytes(lf, op->g.vh)) != cudaSuccess)
       return fail(B200_ENOMEM, "cudaMalloc for links failed");
     B200_CHECK_CUDA(launch_links_from_lex(lf, op->links[lf], op->u_lex, op->g, op->bc, st));
     // the hops fetch links before they wait for earlier kernels (set_config
@@ -315,7 +316,7 @@ int tune_hop(b200_dwf* op, int prec, const HopParams& p0, cudaStream_t st, int* 
     for (int i = 0; i < 2; ++i)
       if (!op->ws->tune_out[i][prec]) {
         const size_t bytes = field_bytes(prec, op->g.vh, op->g.ls);
-        if (cudaMalloc(&op->ws->tune_out[i][prec], bytes) != cudaSuccess) {
+        if (device_malloc(&op->ws->tune_out[i][prec], bytes) != cudaSuccess) {
           op->ws->tune_out[i][prec] = nullptr;
           return fail(B200_ENOMEM, "cudaMalloc for autotuner scratch failed");
         }
@@ -729,9 +730,9 @@ int b200_dwf_create(b200_dwf_t** out, const int lattice[4], int Ls, double mq, d
   int red_n = site_s_grid(Ls, op->g.vh) + hop_grid(Ls, op->g.vh);
   if (op->g.vh <= kSplitMaxSites) red_n += hop_partials(kHopSplit, Ls, op->g.vh);
   op->red_n = red_n;
-  if (cudaMalloc(&op->red, (size_t)red_n * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&op->sc, SC_N * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&op->err, sizeof(int)) != cudaSuccess ||
+  if (device_malloc(&op->red, (size_t)red_n * sizeof(double)) != cudaSuccess ||
+      device_malloc(&op->sc, SC_N * sizeof(double)) != cudaSuccess ||
+      device_malloc(&op->err, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&op->err_host, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&op->sc_host, (SC_N > MS_N ? SC_N : MS_N) * sizeof(double)) != cudaSuccess) {
     b200_dwf_destroy(op);
@@ -788,7 +789,7 @@ size_t b200_dwf_field_nreal(const b200_dwf_t* op) {
 
 static int set_config_common(b200_dwf_t* op, const double* u, cudaMemcpyKind kind, cudaStream_t st) {
   const size_t n = (size_t)18 * 8 * op->g.vh;   // 18 * Nvol * 4
-  if (!op->u_lex && cudaMalloc(&op->u_lex, n * sizeof(double)) != cudaSuccess)
+  if (!op->u_lex && device_malloc(&op->u_lex, n * sizeof(double)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for lexical links failed");
   B200_CHECK_CUDA(cudaMemcpyAsync(op->u_lex, u, n * sizeof(double), kind, st));
   op->have_links = true;
@@ -812,7 +813,7 @@ int b200_field_convert(b200_dwf_t* op, int prec, void* v, const double* w_host, 
   if (!op || !v || !w_host || prec < 0 || prec > 3) return fail(B200_EINVAL, "invalid argument");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t n = b200_dwf_field_nreal(op);
-  if (!op->stage && cudaMalloc(&op->stage, n * sizeof(double)) != cudaSuccess)
+  if (!op->stage && device_malloc(&op->stage, n * sizeof(double)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for the staging field failed");
   B200_CHECK_CUDA(cudaMemcpyAsync(op->stage, w_host, n * sizeof(double), cudaMemcpyHostToDevice, st));
   B200_CHECK_CUDA(launch_from_corelib(prec, v, op->stage, op->g, st));
@@ -827,7 +828,7 @@ static int ring_slot(b200_dwf_t* op, int dir, cudaStream_t st, int* slot) {
   op->ring_next[dir] = (k + 1) % 2;
   if (!op->ring_buf[dir][k]) {
     const size_t bytes = b200_dwf_field_nreal(op) * sizeof(double);
-    if (cudaMalloc(&op->ring_buf[dir][k], bytes) != cudaSuccess) {
+    if (device_malloc(&op->ring_buf[dir][k], bytes) != cudaSuccess) {
       op->ring_buf[dir][k] = nullptr;
       return fail(B200_ENOMEM, "cudaMalloc of %zu bytes for a transfer staging field failed", bytes);
     }
@@ -894,7 +895,7 @@ int b200_field_reverse(b200_dwf_t* op, int prec, double* v_host, const void* w, 
   if (!op || !v_host || !w || prec < 0 || prec > 3) return fail(B200_EINVAL, "invalid argument");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t n = b200_dwf_field_nreal(op);
-  if (!op->stage && cudaMalloc(&op->stage, n * sizeof(double)) != cudaSuccess)
+  if (!op->stage && device_malloc(&op->stage, n * sizeof(double)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for the staging field failed");
   B200_CHECK_CUDA(launch_to_corelib(prec, op->stage, w, op->g, st));
   B200_CHECK_CUDA(cudaMemcpyAsync(v_host, op->stage, n * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1198,11 +1199,11 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
     if ((rc = ensure_work(op, prec, i))) return rc;
   const Geom& g = op->g;
   const int nb_hop = hop_grid(g.ls, g.vh);
-  if (!op->ms_state && cudaMalloc(&op->ms_state, kMsStateSize * sizeof(double)) != cudaSuccess)
+  if (!op->ms_state && device_malloc(&op->ms_state, kMsStateSize * sizeof(double)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for multishift state failed");
-  if (!op->ms_red && cudaMalloc(&op->ms_red, (size_t)kMaxShift * nb_hop * sizeof(double)) != cudaSuccess)
+  if (!op->ms_red && device_malloc(&op->ms_red, (size_t)kMaxShift * nb_hop * sizeof(double)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for multishift partials failed");
-  if (!op->ms_ptrs && cudaMalloc(&op->ms_ptrs, 2 * kMaxShift * sizeof(void*)) != cudaSuccess)
+  if (!op->ms_ptrs && device_malloc(&op->ms_ptrs, 2 * kMaxShift * sizeof(void*)) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for multishift pointers failed");
   // search directions p_i: p_0 is a work slot, the others come from the
   // multishift pool shared by every plan of this field size
@@ -1220,7 +1221,7 @@ int b200_shiftcg_solve(b200_dwf_t* op, void* const* x, const double* sigma, int 
   void* p0s = nullptr;
   std::vector<void*> wp(kMaxWin, nullptr);
   if (window > 0) {
-    if (!op->ms_win_ptrs && cudaMalloc(&op->ms_win_ptrs, kMaxWin * sizeof(void*)) != cudaSuccess)
+    if (!op->ms_win_ptrs && device_malloc(&op->ms_win_ptrs, kMaxWin * sizeof(void*)) != cudaSuccess)
       return fail(B200_ENOMEM, "cudaMalloc for multishift window pointers failed");
     for (int l = 0; l < window; ++l)
       if (ms_pool_slot(op->ws->win, l, fbytes, &wp[l]))
@@ -1523,12 +1524,12 @@ int b200_fcg_solve(b200_dwf_t* op, b200_lp_t* lp, void* x, const void* b, int ma
   const size_t nbuf = 2 * (size_t)(M + 1) + 3;
   while (op->fcg_buf.size() < nbuf) {
     void* q = nullptr;
-    if (cudaMalloc(&q, fb) != cudaSuccess) return fail(B200_ENOMEM, "cudaMalloc for a flexible-CG field failed");
+    if (device_malloc(&q, fb) != cudaSuccess) return fail(B200_ENOMEM, "cudaMalloc for a flexible-CG field failed");
     op->fcg_buf.push_back(q);
   }
-  if (!op->fcg_part && cudaMalloc(&op->fcg_part, sizeof(double2) * zblas_blocks() * kZMaxMulti) != cudaSuccess)
+  if (!op->fcg_part && device_malloc(&op->fcg_part, sizeof(double2) * zblas_blocks() * kZMaxMulti) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for flexible-CG partials failed");
-  if (!op->fcg_sc && cudaMalloc(&op->fcg_sc, sizeof(double2) * 32) != cudaSuccess)
+  if (!op->fcg_sc && device_malloc(&op->fcg_sc, sizeof(double2) * 32) != cudaSuccess)
     return fail(B200_ENOMEM, "cudaMalloc for flexible-CG scalars failed");
   void** P = op->fcg_buf.data();
   void** Q = op->fcg_buf.data() + (M + 1);

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 #include "dwf_kernels.h"
 #include "su3_lex.cuh"
 
@@ -345,12 +346,19 @@ int fail_code(int code, const char* msg) {
 // allocations from a pool of this library, one per device, so that calls on
 // several streams and threads each have their own and a repeated call does
 // not wait for the allocator.  At most kPoolKeep bytes stay with the pool
-// between calls; gauge_scratch_trim (run when a plan is destroyed) gives them
-// back.
+// between calls.  They go back to the device when a plan is destroyed, when
+// b200_scratch_release asks for it and when an allocation of this library
+// would fail without them.
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kPoolKeep = 2ull << 30;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
+bool g_pool_keeps[kMaxDevices] = {};      // the release threshold is kPoolKeep (else 0)
+
+cudaError_t pool_keep(int dev, unsigned long long bytes) {
+  g_pool_keeps[dev] = bytes != 0;
+  return cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &bytes);
+}
 
 cudaMemPool_t scratch_pool() {
   int dev = 0;
@@ -361,23 +369,42 @@ cudaMemPool_t scratch_pool() {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    unsigned long long keep = kPoolKeep;
     if (cudaMemPoolCreate(&g_pool[dev], &props) != cudaSuccess) {
       cudaGetLastError();
       g_pool[dev] = nullptr;
-    } else {
-      cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
     }
   }
+  if (g_pool[dev] && !g_pool_keeps[dev]) pool_keep(dev, kPoolKeep);
   return g_pool[dev];
 }
 
 }  // namespace
 
+// What no call uses any more goes back at once; with the threshold at 0 (until
+// the next gauge force) what a call still in flight frees goes back at the next
+// synchronisation.
 void gauge_scratch_trim() {
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  for (int d = 0; d < kMaxDevices; ++d)
-    if (g_pool[d]) cudaMemPoolTrimTo(g_pool[d], 0);
+  // no stream is touched: safe while this thread captures one
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    for (int d = 0; d < kMaxDevices; ++d)
+      if (g_pool[d]) {
+        pool_keep(d, 0);
+        cudaMemPoolTrimTo(g_pool[d], 0);
+      }
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
+cudaError_t device_malloc_bytes(void** p, size_t n) {
+  const cudaError_t e = cudaMalloc(p, n);
+  if (e != cudaErrorMemoryAllocation) return e;
+  gauge_scratch_trim();
+  const cudaError_t e2 = cudaMalloc(p, n);
+  if (e2 == cudaSuccess) cudaGetLastError();    // the first failure is over
+  return e2;
 }
 
 cudaError_t launch_links_to_planar(double2* out, const double* u, size_t vol, cudaStream_t st) {
@@ -390,6 +417,11 @@ cudaError_t launch_links_to_planar(double2* out, const double* u, size_t vol, cu
 using namespace b200;
 
 extern "C" {
+
+int b200_scratch_release(void) {
+  gauge_scratch_trim();
+  return 0;
+}
 
 int b200_gauge_force_rect(const int lattice[4], double beta, double c_plaq, double c_rect, double* force,
                           const double* u, void* stream) {
@@ -430,7 +462,7 @@ int b200_gauge_action_rect(const int lattice[4], double beta, double c_plaq, dou
   cudaStream_t st = (cudaStream_t)stream;
   const int nb = (int)((g.vol + 255) / 256);
   double* part = nullptr;
-  G_CHECK(cudaMalloc(&part, sizeof(double) * 2 * nb));
+  G_CHECK(device_malloc(&part, sizeof(double) * 2 * nb));
   gauge_action_kernel<<<nb, 256, 0, st>>>(u, g, part);
   std::vector<double> h(2 * (size_t)nb);
   cudaError_t e = cudaGetLastError();
@@ -468,7 +500,7 @@ int b200_momentum_energy(const int lattice[4], const double* ip, double* H, void
   cudaStream_t st = (cudaStream_t)stream;
   const int nb = 592;
   double* part = nullptr;
-  G_CHECK(cudaMalloc(&part, sizeof(double) * nb));
+  G_CHECK(device_malloc(&part, sizeof(double) * nb));
   norm2_links_kernel<<<nb, 256, 0, st>>>(ip, 18 * 4 * g.vol, part);
   std::vector<double> h(nb);
   cudaError_t e = cudaGetLastError();

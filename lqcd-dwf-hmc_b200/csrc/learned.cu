@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 #include "dwf_hop.cuh"
 #include "learned.h"
 #include "umma.cuh"
@@ -972,13 +973,13 @@ int ensure_train_buffers(b200_lp* lp) {
   for (int i = Y3; i < NACT; ++i) {
     if (lp->act[i]) continue;
     const int ch = (i == Y3 || i == D3 || i == T4 || i == AD4) ? kLpIn : lp->hidden;
-    if (cudaMalloc(&lp->act[i], act_bytes(lp, ch)) != cudaSuccess) {
+    if (device_malloc(&lp->act[i], act_bytes(lp, ch)) != cudaSuccess) {
       lp->act[i] = nullptr;
       return lp_fail(B200_ENOMEM, "allocation of the training buffers failed");
     }
   }
   if (!lp->partial &&
-      cudaMalloc(&lp->partial, sizeof(float2) * (size_t)lp->max_blocks * kLpPaths * lp->hidden * lp->hidden) !=
+      device_malloc(&lp->partial, sizeof(float2) * (size_t)lp->max_blocks * kLpPaths * lp->hidden * lp->hidden) !=
           cudaSuccess) {
     lp->partial = nullptr;
     return lp_fail(B200_ENOMEM, "allocation of the gradient partials failed");
@@ -1045,15 +1046,15 @@ int b200_lp_create(b200_lp_t** out, b200_dwf_t* op, int hidden, unsigned long lo
           w[E] = make_float2((float)(nr + ((path == 0 && a == b) ? 1.0 : 0.0)), (float)ni);
         }
   const size_t pb = sizeof(float2) * lp->nparam;
-  bool ok = cudaMalloc(&lp->master, pb) == cudaSuccess && cudaMalloc(&lp->adam_m, pb) == cudaSuccess &&
-            cudaMalloc(&lp->adam_v, pb) == cudaSuccess && cudaMalloc(&lp->grad, pb) == cudaSuccess &&
-            cudaMalloc(&lp->wf, pb) == cudaSuccess && cudaMalloc(&lp->wadj, pb) == cudaSuccess;
+  bool ok = device_malloc(&lp->master, pb) == cudaSuccess && device_malloc(&lp->adam_m, pb) == cudaSuccess &&
+            device_malloc(&lp->adam_v, pb) == cudaSuccess && device_malloc(&lp->grad, pb) == cudaSuccess &&
+            device_malloc(&lp->wf, pb) == cudaSuccess && device_malloc(&lp->wadj, pb) == cudaSuccess;
   // the forward pass needs the hidden layers' activations only; the
   // training buffers come with the first training call
-  for (int i = Y1E; ok && i <= Y2O; ++i) ok = cudaMalloc(&lp->act[i], act_bytes(lp, hidden)) == cudaSuccess;
+  for (int i = Y1E; ok && i <= Y2O; ++i) ok = device_malloc(&lp->act[i], act_bytes(lp, hidden)) == cudaSuccess;
   lp->max_blocks = 148 * 3;
-  ok = ok && cudaMalloc(&lp->red, sizeof(double) * kRedBlocks) == cudaSuccess;
-  ok = ok && cudaMalloc(&lp->sc, sizeof(double) * 4) == cudaSuccess;
+  ok = ok && device_malloc(&lp->red, sizeof(double) * kRedBlocks) == cudaSuccess;
+  ok = ok && device_malloc(&lp->sc, sizeof(double) * 4) == cudaSuccess;
   ok = ok && cudaMallocHost(&lp->sc_host, sizeof(double) * 4) == cudaSuccess;
   if (!ok) {
     b200_lp_destroy(lp);

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 
 namespace b200 {
 void set_last_error(int code, const char* fmt, ...);
@@ -261,7 +262,7 @@ int b200_rng_create(b200_rng_t** out, const int lattice[4], unsigned long seed) 
   b200_rng* g = new b200_rng();
   for (int mu = 0; mu < 4; ++mu) g->L[mu] = lattice[mu];
   g->nplanes = lattice[2] * lattice[3];
-  if (cudaMalloc(&g->state, (size_t)g->nplanes * kStride * sizeof(int)) != cudaSuccess) {
+  if (b200::device_malloc(&g->state, (size_t)g->nplanes * kStride * sizeof(int)) != cudaSuccess) {
     delete g;
     return rng_fail(B200_ENOMEM, "cudaMalloc for the generator state failed");
   }

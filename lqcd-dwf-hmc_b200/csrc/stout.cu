@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/b200dwf.h"
+#include "device_alloc.h"
 #include "dwf_kernels.h"
 #include "su3_lex.cuh"
 
@@ -412,7 +413,7 @@ int b200_smear_create(b200_smear_t** out, const int lattice[4], double rho, int 
   cudaGetDevice(&sm->device);
   const size_t n = nreal_cfg(sm) / 2;      // double2 of one field
   const size_t fields = nsmear > 0 ? nsmear + 3 : 1;
-  if (sm->g.vol > 0x7fffffffu || cudaMalloc(&sm->block, fields * n * sizeof(double2)) != cudaSuccess) {
+  if (sm->g.vol > 0x7fffffffu || device_malloc(&sm->block, fields * n * sizeof(double2)) != cudaSuccess) {
     sm->block = nullptr;
     b200_smear_destroy(sm);
     set_last_error(B200_ENOMEM, "smear_create: device allocation failed");
@@ -504,7 +505,7 @@ static int make_lex(b200_smear* sm, int level) {
   double* buf = nullptr;
   cudaStream_t st = nullptr;
   cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&buf, nreal_cfg(sm) * sizeof(double));
+  if (e == cudaSuccess) e = device_malloc(&buf, nreal_cfg(sm) * sizeof(double));
   if (e == cudaSuccess) {
     planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(buf, planar_level(sm, level));
     e = cudaGetLastError();
