@@ -33,10 +33,15 @@ constexpr int kMaxLs = 32;
 // ---------------------------------------------------------------- launch overlap
 // The kernels of an operator application or a solver iteration follow one
 // another on the same fields, and on small lattices the launch and first
-// instructions of each took a quarter of its time.  A kernel first lets the
-// next one launch, does what depends on its parameters alone (index
-// arithmetic, L2 requests for the links), and waits here for the kernels
-// before it to have finished and their writes to be visible.
+// instructions of each took a quarter of its time.  A kernel does what depends
+// on its parameters alone (index arithmetic, L2 requests, fetching links, which
+// are complete before any launch that reads them), waits here for the kernels
+// before it to have finished and their writes to be visible, and then lets the
+// next one launch.  With that permission given before the wait, on grids of
+// about a wave the blocks of several later kernels took places on the SMs and
+// those of the kernel at work were spread unevenly: DdagD in a CUDA graph, FP64
+// 8^3x16 Ls=4 49.0 us against 22.0, 8^4 Ls=8 31.5 against 20.2, f16 8^3x16 Ls=8
+// 31.4 against 21.7; with several waves the order makes no difference.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

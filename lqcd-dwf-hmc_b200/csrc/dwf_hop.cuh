@@ -615,7 +615,6 @@ template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
   using LSt = LinkStage<LS, LF>;
-  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), !LSt::on);
   using St = Store<P>;
   using R = typename St::R;
@@ -679,6 +678,7 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
     }
   }
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) {
     async_copy_wait();
     return;
@@ -768,8 +768,8 @@ __device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, 
 template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_split_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -925,9 +925,9 @@ __device__ __forceinline__ void reconstruct_acc2(float2* acc, const float2* o, f
 template <int LS, int P, int LF, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_pair_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), true);
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -1129,9 +1129,9 @@ __device__ __forceinline__ void pair_compute(const PairRaw<P>& r, float ph, floa
 template <int LS, int P, int EPI, int FK, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_pair_pf_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   hop_prefetch<LS, P, LINK_F16_18>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), true);
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -1268,9 +1268,9 @@ template <int LS, int P, int LF, int GS = 32 / LS> struct TmaGeom {
 template <int LS, int P, int LF, int EPI, int FK, int S, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_tma_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (32 / LS)), 4 * (32 / LS), false);
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -1442,9 +1442,9 @@ dwf_hop_tma_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename
 template <int LS, int P, int LF, int EPI, int FK, int S, int MB>
 __global__ void __launch_bounds__(128, MB)
 dwf_hop_tma_pair_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   hop_prefetch<LS, P, LF>(p, p.site0 + blockIdx.x * (4 * (64 / LS)), 4 * (64 / LS), false);
   pdl_wait();
+  pdl_launch_dependents();
   if (p.skip && *p.skip != 0.0) return;
   using St = Store<P>;
   using R = typename St::R;

@@ -132,7 +132,9 @@ cudaError_t launch_force(const ForceParams& p, cudaStream_t st);
 
 // Launch with programmatic stream serialisation: the kernel may start while
 // the one before it in the stream drains; it runs pdl_wait() (dwf_common.cuh)
-// before it touches anything an earlier kernel wrote or reads.
+// before it touches anything an earlier kernel wrote or reads.  Links are the
+// one exception: the hops may fetch them before, since the host waits for their
+// conversion (set_config, and the first use of a link format).
 template <typename... KA, typename... A>
 cudaError_t launch_pdl(void (*kernel)(KA...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchAttribute attr[1];

@@ -84,8 +84,8 @@ template <int LS, int P, int OPA, int OPB>
 __global__ void __launch_bounds__(128)
 sop_kernel(SopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k,
            const __grid_constant__ ChainCoef<typename Store<P>::R> kee) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   using St = Store<P>;
   using R = typename St::R;
   constexpr int G = 32 / LS;
@@ -228,8 +228,8 @@ cudaError_t launch_sop(int prec, const SopParams& p, const ChainCoefs& c, cudaSt
 template <int LS, int P>
 __global__ void __launch_bounds__(128)
 cg_update_kernel(CgUpdParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (*p.done >= 2.0) return;
   using St = Store<P>;
   using R = typename St::R;
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(128)
 ms_update_kernel(MsUpdParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
   using St = Store<P>;
   using R = typename St::R;
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (p.st[MS_DONE] != 0.0) return;   // solve finished: replayed iteration is a no-op
   constexpr int G = 32 / LS;
   constexpr int WARPS = 4;
@@ -459,8 +459,8 @@ __device__ double block_sum_partials(const double* partials, int n) {
 }
 
 __global__ void ms_scalar_kernel(int step, const double* partials, int n, double* st, int nshift) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (st[MS_DONE] != 0.0) return;     // solve finished: a replayed iteration is a no-op
   double* zeta1 = st + MS_N + MSA_ZETA1 * kMaxShift;
   double* zeta2 = st + MS_N + MSA_ZETA2 * kMaxShift;
@@ -564,8 +564,8 @@ __device__ __forceinline__ bool ms_window_due(const double* st) {
 // p_i = PC0 p_i + sum_l PC_l r_l ; x_i += XC0 p_i(old) + sum_l XC_l r_l for
 // every shift active in the window; flat over the FP64 field as double2.
 __global__ void __launch_bounds__(256) ms_flush_kernel(MsUpdParams p, long n2) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const double* st = p.st;
   if (!ms_window_due(st)) return;
   __shared__ double cs[2 * kMaxShift * (kMaxWin + 1)];
@@ -630,8 +630,8 @@ __global__ void __launch_bounds__(256) ms_flush_kernel(MsUpdParams p, long n2) {
 }
 
 __global__ void ms_window_reset_kernel(double* st) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (threadIdx.x != 0 || !ms_window_due(st)) return;
   for (int i = 0; i < kMaxShift; ++i) {
     double* pc = st + kMsCoef + i * (kMaxWin + 1);
@@ -837,8 +837,8 @@ size_t link_bytes(int lf, size_t vh) {
 }
 
 __global__ void finalize_kernel(const double* partials, int n, double* out, int op) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   __shared__ double ws[32];
   if (op != FIN_SUM && out[SC_DONE] != 0.0) {       // a CG that is over
     if (threadIdx.x == 0 && op == FIN_CG_ALPHA && out[SC_DONE] == 1.0) out[SC_DONE] = 2.0;
