@@ -1047,12 +1047,12 @@ __device__ __forceinline__ void pair_fetch(const HopParams& p, int nb, size_t li
   const uint4* c = reinterpret_cast<const uint4*>(colp);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    r.c0[k] = __ldg(c + k * LS + s0);
-    r.c1[k] = __ldg(c + k * LS + s1);
+    r.c0[k] = ld_field(c + k * LS + s0);
+    r.c1[k] = ld_field(c + k * LS + s1);
   }
   const float* scp = reinterpret_cast<const float*>(c + 3 * LS);
-  r.sc0 = __ldg(scp + s0);
-  r.sc1 = __ldg(scp + s1);
+  r.sc0 = ld_field(scp + s0);
+  r.sc1 = ld_field(scp + s1);
   const uint4* lp = reinterpret_cast<const uint4*>(p.links) + lidx * 3;
   r.l0 = __ldg(lp);
   r.l1 = __ldg(lp + 1);
