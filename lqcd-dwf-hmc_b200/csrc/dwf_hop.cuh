@@ -598,7 +598,15 @@ template <int LS, int LF> struct LinkStage {
   static constexpr bool on = LF == LINK_F64_18;
   static constexpr int G = 32 / LS;
   static constexpr int records = G * 8;
-  static constexpr int bytes = on ? records * (144 + 4) : 0;       // records, then their indices
+  // 16-byte chunks from one site's records to the next: one more than the 72
+  // that they take, since 72 chunks are a multiple of 128 bytes and the G
+  // sites' reads of one entry would all meet in the same four banks.  DdagD
+  // FP64 16^3x32 in us (fastest direct budget), links from global memory / staged
+  // without the extra chunk / with it: Ls 4 245 / 296 / 243, Ls 6 351 / 380 /
+  // 324, Ls 8 395 / 371 / 352; at Ls 12 and 16 (two sites a warp) no difference.
+  static constexpr int site_chunks = 8 * 9 + 1;
+  static constexpr int index_at = G * site_chunks * 16;            // the records' indices, after them
+  static constexpr int bytes = on ? index_at + records * 4 : 0;
 };
 
 // Bytes of shared memory per warp of the direct kernel: the staged links and,
@@ -659,7 +667,7 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
     nb[7] = (t == 0) ? site + (p.nt - 1) * st4 : site - st4;
   }
   if constexpr (LSt::on) {
-    unsigned int* rec = reinterpret_cast<unsigned int*>(wbase + LSt::records * 144);
+    unsigned int* rec = reinterpret_cast<unsigned int*>(wbase + LSt::index_at);
     // record of direction d: forward U_mu(x) of this parity, backward
     // U_mu(x-mu) of the other; past the last site, record 0 (never used)
     if (g < G) {
@@ -674,7 +682,8 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
     const uint32_t dst = smem_u32(wbase);
     for (int i = lane; i < LSt::records * 9; i += 32) {
       const int r = i / 9;
-      async_copy16(dst + i * 16, reinterpret_cast<const unsigned char*>(p.links) + (size_t)rec[r] * 144 + (i - 9 * r) * 16);
+      async_copy16(dst + (i + r / 8) * 16,
+                   reinterpret_cast<const unsigned char*>(p.links) + (size_t)rec[r] * 144 + (i - 9 * r) * 16);
     }
   }
   pdl_wait();
@@ -687,7 +696,7 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
   R acc[24];
 #pragma unroll
   for (int i = 0; i < 24; ++i) acc[i] = 0;
-  const double2* lrec = reinterpret_cast<const double2*>(wbase) + (g < G ? g : 0) * 8 * 9;
+  const double2* lrec = reinterpret_cast<const double2*>(wbase) + (g < G ? g : 0) * LSt::site_chunks;
 
 #define B200_HOP_HALF(D, MU, SIGN, EDGE)                                             \
   {                                                                                  \
