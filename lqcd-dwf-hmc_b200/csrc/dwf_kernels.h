@@ -147,7 +147,10 @@ cudaError_t launch_pdl(void (*kernel)(KA...), int grid, int block, size_t smem, 
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  // the caller reports it; left set, the next plain launch would report it too
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // number of blocks the reductions of each launcher produce
