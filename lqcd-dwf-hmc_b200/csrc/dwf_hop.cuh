@@ -747,8 +747,9 @@ dwf_hop_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Sto
 // and computes their two hops, the partial results meet in shared memory (a
 // quarter of the components summed by each warp) and warp 0 runs the
 // epilogue.  The autotuner picks it where it is the fastest, up to the plan's
-// kSplitMaxSites.  DdagD in FP64, 4^3x8 Ls=8 (four hops, synchronous call): 50.7
-// -> 40.1 us.
+// kSplitMaxBlocks.  DdagD FP64 4^3x8 Ls=8, four hops in a CUDA graph: 17.5 us with
+// the direct kernels, 14.5 so.  (A second budget of 4 resident blocks gained only
+// where the direct kernels are ahead of both.)
 template <typename R, int P, int LS, int LF, int MU, bool kDagHop>
 __device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, int nbp, int nbm, bool lastp,
                                            bool firstm, R* acc) {
@@ -774,8 +775,8 @@ __device__ __forceinline__ void split_axis(const HopParams& p, int s, int site, 
   reconstruct_acc<R, MU, -1, kPh>(acc, o, (kPh || !firstm) ? R(1) : (R)p.bc[MU]);
 }
 
-template <int LS, int P, int LF, int EPI, int FK, int MB>
-__global__ void __launch_bounds__(128, MB)
+template <int LS, int P, int LF, int EPI, int FK>
+__global__ void __launch_bounds__(128, 2)
 dwf_hop_split_kernel(const HopParams p, const __grid_constant__ ChainCoef<typename Store<P>::R> k) {
   pdl_wait();
   pdl_launch_dependents();

@@ -155,7 +155,7 @@ cudaError_t launch_pdl(void (*kernel)(KA...), int grid, int block, size_t smem, 
 
 // number of blocks the reductions of each launcher produce
 int hop_grid(int ls, int vh);
-constexpr int kHopSplit = 10, kHopSplit4 = 11;   // the hop variants whose blocks hold one warp's sites
+constexpr int kHopSplit = 10;    // the hop variant whose blocks hold one warp's sites
 int hop_partials(int variant, int ls, int vh);   // |o1|^2 partials of a hop launch
 int site_s_grid(int ls, int vh);
 constexpr int kSiteSBlock = 128;

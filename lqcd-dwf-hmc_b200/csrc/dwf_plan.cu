@@ -277,20 +277,24 @@ SopParams sop_base(const b200_dwf* op) {
 // B200_AUTOTUNE=0 disables tuning (variant 0).  The first call of a
 // combination must not be inside a CUDA graph capture.
 typedef std::tuple<int, int, int, int, int> TuneKey;   // vh, ls, prec, epi, fk
-constexpr int kHopVariants = 12;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
+constexpr int kHopVariants = 11;   // direct, TMA 2-stage, TMA 3-stage, TMA 2-stage + direct at
                                   // higher occupancy, packed two-slice FP32x2 (direct, TMA),
                                   // 4-deep TMA, packed with all directions in flight, packed
                                   // half-storage with register prefetch, the four axes on
-                                  // four warps (two register budgets)
-// The split kernel's range: at 256 sites (4^3x8, Ls 8) it takes DdagD from 50.7
-// to 40.1 us; at 2,048 it is level with the direct kernels (FP64 D_eo^+ Ls 8:
-// 8.5 against 8.6 us, Ls 12: 9.1 against 8.6), at 4,096 every SM has several
-// blocks and it is the slower one (Ls 12: 14.7 against 9.7 us, at 13,824 sites
-// 44.6 against 28.4).  Its block partials fit the plan's buffer up to here.
-constexpr int kSplitMaxSites = 2048;
+                                  // four warps
+// The split kernel's range: as long as each of its blocks has an SM to itself.
+// DdagD in a CUDA graph, fastest direct kernel / split, in us: 64 blocks (4^3x8
+// Ls 8) FP64 17.5 / 14.5, f16 18.6 / 15.3; 128 blocks (4^2x8^2 Ls 8) 17.7 / 16.6,
+// 18.7 / 17.9; from 173 blocks on (6^3x8 Ls 6) level, 19.3 / 19.8, 18.8 / 19.2;
+// 432 (6^3x8 Ls 12) 18.8 / 29.5, 1024 (8^4 Ls 12) 25.3 / 50.7.  (One hop launched
+// again and again gains up to 256 blocks, 3.6 / 3.3, which is what the autotuner
+// times, so the limit is here.)  Its block partials fit the plan's buffer up to
+// here.
+constexpr int kSplitMaxBlocks = 148;
+bool split_fits(int ls, int vh) { return hop_partials(kHopSplit, ls, vh) <= kSplitMaxBlocks; }
 
 bool variant_supported(int prec, int ls, int vh, int v) {
-  if (v == kHopSplit || v == kHopSplit4) return vh <= kSplitMaxSites;
+  if (v == kHopSplit) return split_fits(ls, vh);
   if (v < 5) return true;
   if (v == 7 && prec == PREC_F64) return true;
   if (v == 9 && (prec == PREC_F64 || prec == PREC_F32)) return false;
@@ -728,7 +732,7 @@ int b200_dwf_create(b200_dwf_t** out, const int lattice[4], int Ls, double mq, d
     }
   }
   int red_n = site_s_grid(Ls, op->g.vh) + hop_grid(Ls, op->g.vh);
-  if (op->g.vh <= kSplitMaxSites) red_n += hop_partials(kHopSplit, Ls, op->g.vh);
+  if (split_fits(Ls, op->g.vh)) red_n += hop_partials(kHopSplit, Ls, op->g.vh);
   op->red_n = red_n;
   if (device_malloc(&op->red, (size_t)red_n * sizeof(double)) != cudaSuccess ||
       device_malloc(&op->sc, SC_N * sizeof(double)) != cudaSuccess ||

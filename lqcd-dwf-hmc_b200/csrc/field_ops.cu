@@ -19,7 +19,7 @@ int hop_grid(int ls, int vh) {
 }
 
 int hop_partials(int variant, int ls, int vh) {
-  return variant == kHopSplit || variant == kHopSplit4 ? hop_split_grid(ls, vh) : hop_grid(ls, vh);
+  return variant == kHopSplit ? hop_split_grid(ls, vh) : hop_grid(ls, vh);
 }
 
 int site_s_grid(int ls, int vh) {

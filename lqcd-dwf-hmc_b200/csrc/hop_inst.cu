@@ -100,12 +100,12 @@ cudaError_t run_tma_pair(const HopParams& p, const ChainCoefs& c, cudaStream_t s
   return launch_pdl(k, hop_pair_grid(LS, p.site_end - p.site0), 128, smem, st, p, kc);
 }
 
-template <int LS, int P, int EPI, int FK, int MB>
+template <int LS, int P, int EPI, int FK>
 cudaError_t run_split(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
   using R = typename Store<P>::R;
   constexpr int LF = DefaultLink<P>::v;
   constexpr size_t smem = hop_split_smem_bytes<LS, P>();
-  auto k = dwf_hop_split_kernel<LS, P, LF, EPI, FK, MB>;
+  auto k = dwf_hop_split_kernel<LS, P, LF, EPI, FK>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -126,11 +126,10 @@ cudaError_t run_split(const HopParams& p, const ChainCoefs& c, cudaStream_t st) 
 // with all 8 directions in flight at once; 9: the packed kernel for f16/bf16
 // storage fetching the next direction into registers while computing the
 // current one (5-9 packed: FP32 arithmetic only); 10: the four axes on four
-// warps, for small lattices; 11: the same at 4 resident blocks.
+// warps, for small lattices.
 template <int LS, int P, int EPI, int FK>
 cudaError_t run(const HopParams& p, const ChainCoefs& c, cudaStream_t st) {
-  if (p.variant == kHopSplit) return run_split<LS, P, EPI, FK, 2>(p, c, st);
-  if (p.variant == kHopSplit4) return run_split<LS, P, EPI, FK, 4>(p, c, st);
+  if (p.variant == kHopSplit) return run_split<LS, P, EPI, FK>(p, c, st);
   if (p.variant == 1) return run_tma<LS, P, EPI, FK, 2, 1>(p, c, st);
   if (p.variant == 2) return run_tma<LS, P, EPI, FK, 3, 1>(p, c, st);
   if (p.variant == 3) return run_tma<LS, P, EPI, FK, 2, HopMinBlocks<P>::v1>(p, c, st);

@@ -19,15 +19,18 @@ CASES = [
     ([6, 4, 2, 6], 12, 1.5, 0.5, (1, 1, -1, 1)),
     ([4, 2, 6, 4], 16, 1.0, 0.0, (1, 1, 1, -1)),
 ]
-# FP64 rounding of a few thousand operations; FP32 likewise; half storage rounds
-# every intermediate field (2^-11, 2^-8) four times
-TOL = {0: 1e-13, 1: 5e-6, 2: 5e-3, 3: 4e-2}
+# FP64 rounding of a few thousand operations; FP32 likewise.  Half storage rounds
+# the input and up to four fields after it by at most 2^-12 (2^-9) of a slice's
+# largest component, about three times their root mean square, uniformly (1 /
+# sqrt 3 of it): 4.2e-4 (3.4e-3) each, times sqrt 5 and 1.7 for M_ee^-1.
+TOL = {0: 1e-13, 1: 5e-6, 2: 1.6e-3, 3: 1.3e-2}
 
 
-# 10, 11: the split kernel at its two register budgets; 0, 4: the direct kernel,
+# 10: the split kernel (every case has at most one block an SM, its range); 0,
+# 4: the direct kernel,
 # whose FP64 links a warp stages for all its sites (at Ls 4 more of them than
 # the epilogue's tile takes, at Ls 4 and 6 fewer lanes per site than directions)
-@pytest.mark.parametrize("variant", ["10", "11", "0", "4"])
+@pytest.mark.parametrize("variant", ["10", "0", "4"])
 @pytest.mark.parametrize("ci", range(len(CASES)))
 def test_split_and_direct_hops_against_oracle(ci, variant, monkeypatch):
     import b200dwf
