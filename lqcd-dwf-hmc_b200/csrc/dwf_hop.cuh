@@ -544,13 +544,16 @@ __device__ __forceinline__ void hop_epilogue(const HopParams& p, const ChainCoef
 }
 
 // The block's streams that come from HBM rather than L2, requested at its
-// start: its sites' link records (each used once by a hop, so every direction
-// would otherwise wait for one), the columns at t+1 (the first touch of a
-// column in a sweep over the sites) and the epilogue's operands.  One thread
-// asks for one run of N consecutive sites; the runs ignore the wrap at the
-// lattice's edges (a hint, never needed for the result) and stay in bounds.
-// Direct FP64 hops at 24^3x48 Ls=16: 895 -> 790 us (D_eo^+), 911 -> 853 us
-// (LU-chain epilogue).
+// start: the epilogue's operands and, with `links` (the kernels that load links
+// and columns as they go: direct in FP32 and half storage, packed), its sites'
+// link records, each used once by a hop, so that every direction would
+// otherwise wait for one, and the columns at t+1, the first touch of a column
+// in a sweep over the sites.  The kernels that fetch both ahead anyway (direct
+// FP64, bulk copies) ask for the operands alone, the split kernel for nothing.
+// One thread asks for one run of N consecutive sites; the runs ignore the wrap
+// at the lattice's edges (a hint, never needed for the result) and stay in
+// bounds.  DdagD 16^3x32 without / with: f32 Ls=16 402 / 348 us (packed), 396 /
+// 341 (direct); FP64 Ls=12 640 / 610 (direct, operands alone).
 template <int LS, int P, int LF>
 __device__ __forceinline__ void hop_prefetch(const HopParams& p, int first, int n, bool links) {
   constexpr int COL = (int)Store<P>::col_bytes(LS);
@@ -590,7 +593,7 @@ template <> struct HopMinBlocks<PREC_BF16> { static constexpr int v0 = 4, v1 = 6
 // 16-byte load of a link costs the L1 data pipe five of its cycles from global
 // memory and under three from shared memory; with nine of them per direction
 // they were over a third of the direct hop's L1 work, which at 77 % busy
-// bounded it.  The warp fetches the 8 records of each of its G sites at its
+// bounded it (62 % now).  The warp fetches the 8 records of each of its G sites at its
 // start, whole lines at a time.  FP64, with the budget of 4 resident blocks now
 // almost free of spills: force 24^3x48 Ls=16 (three hops of 5.5 ms) 5.50 ->
 // 5.21 ms, DdagD Moebius 14x10x6x18 Ls=12 116.8 -> 104.3 us.
