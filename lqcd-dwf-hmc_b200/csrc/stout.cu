@@ -15,7 +15,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/b200dwf.h"
@@ -492,32 +494,50 @@ int b200_smear_set_config(b200_smear_t* sm, const double* u, int on_device, void
   return 0;
 }
 
-// A lexical copy of a level below the top, made on the first request: on the
-// plan's device, whichever the calling thread has current, and on a stream of
-// its own, so that a capture or work in progress on the caller's streams is
-// not touched (the levels are complete when set_config returns).
-static int make_lex(b200_smear* sm, int level) {
-  int current = sm->device;
-  cudaGetDevice(&current);
-  if (current != sm->device) B200_SMEAR_CHECK(cudaSetDevice(sm->device));
+// The plan's device, whichever the calling thread has current, and a capture
+// mode in which allocations do not disturb a capture in progress.
+struct OnPlanDevice {
+  int plan, current;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  double* buf = nullptr;
+  explicit OnPlanDevice(const b200_smear* sm) : plan(sm->device), current(sm->device) {
+    cudaGetDevice(&current);
+    if (current != plan) cudaSetDevice(plan);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  ~OnPlanDevice() {
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (current != plan) cudaSetDevice(current);
+  }
+};
+
+// Planar level -> lexical `out`, on a stream of its own, so that work in
+// progress on the caller's streams is not touched (the levels are complete when
+// set_config returns).
+static cudaError_t level_to_lex(const b200_smear* sm, int level, double* out) {
   cudaStream_t st = nullptr;
   cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = device_malloc(&buf, nreal_cfg(sm) * sizeof(double));
-  if (e == cudaSuccess) {
-    planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(buf, planar_level(sm, level));
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  }
-  if (st) cudaStreamDestroy(st);
-  if (e != cudaSuccess) cudaFree(buf);
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (current != sm->device) cudaSetDevice(current);
+  if (e != cudaSuccess) return e;
+  planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(out, planar_level(sm, level));
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  return e;
+}
+
+static int smear_fail(cudaError_t e, const char* what) {
+  set_last_error(e == cudaErrorMemoryAllocation ? B200_ENOMEM : B200_ECUDA, "%s: %s", what, cudaGetErrorString(e));
+  return e == cudaErrorMemoryAllocation ? B200_ENOMEM : B200_ECUDA;
+}
+
+// The lexical copy of a level below the top that stays with the plan.
+static int make_lex(b200_smear* sm, int level) {
+  OnPlanDevice on(sm);
+  double* buf = nullptr;
+  cudaError_t e = device_malloc(&buf, nreal_cfg(sm) * sizeof(double));
+  if (e == cudaSuccess) e = level_to_lex(sm, level, buf);
   if (e != cudaSuccess) {
-    set_last_error(e == cudaErrorMemoryAllocation ? B200_ENOMEM : B200_ECUDA, "smear_config: %s", cudaGetErrorString(e));
-    return B200_ECUDA;
+    cudaFree(buf);
+    return smear_fail(e, "smear_config");
   }
   sm->lex[level] = buf;
   return 0;
@@ -530,11 +550,43 @@ const double* b200_smear_config(b200_smear_t* sm, int level) {
   return sm->lex[level];
 }
 
+// A level that has no lexical copy goes through one that is given back, or,
+// where there is no room for it, is put in order on the host: the plan keeps no
+// memory for this call, and later set_config calls do no more work after it.
+static int planar_to_host(b200_smear* sm, int level, double* host_out) {
+  OnPlanDevice on(sm);
+  const size_t bytes = nreal_cfg(sm) * sizeof(double), vol = sm->g.vol;
+  double* lex = nullptr;
+  cudaError_t e = device_malloc(&lex, bytes);
+  if (e == cudaSuccess) {
+    e = level_to_lex(sm, level, lex);
+    if (e == cudaSuccess) e = cudaMemcpy(host_out, lex, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(lex);
+    return e == cudaSuccess ? 0 : smear_fail(e, "smear_get_config");
+  }
+  if (e != cudaErrorMemoryAllocation) return smear_fail(e, "smear_get_config");
+  cudaGetLastError();
+  double2* planar = new (std::nothrow) double2[36 * vol];
+  if (!planar) return smear_fail(cudaErrorMemoryAllocation, "smear_get_config");
+  e = cudaMemcpy(planar, planar_level(sm, level).p, bytes, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    for (size_t mu = 0; mu < 4; ++mu)
+      for (size_t site = 0; site < vol; ++site)
+        for (size_t k = 0; k < 9; ++k)
+          memcpy(host_out + 18 * (site + vol * mu) + 2 * k, planar + (9 * mu + k) * vol + site, sizeof(double2));
+  delete[] planar;
+  return e == cudaSuccess ? 0 : smear_fail(e, "smear_get_config");
+}
+
 int b200_smear_get_config(b200_smear_t* sm, int level, double* host_out, void* stream) {
-  const double* src = b200_smear_config(sm, level);
-  if (!src || !host_out) { set_last_error(B200_EINVAL, "smear_get_config: invalid level or no config"); return B200_EINVAL; }
+  if (!sm || !host_out || level < 0 || level > sm->nsmear || !sm->have_config) {
+    set_last_error(B200_EINVAL, "smear_get_config: invalid level or no config");
+    return B200_EINVAL;
+  }
   cudaStream_t st = (cudaStream_t)stream;
-  B200_SMEAR_CHECK(cudaMemcpyAsync(host_out, src, nreal_cfg(sm) * sizeof(double), cudaMemcpyDeviceToHost, st));
+  std::lock_guard<std::mutex> lock(sm->mu);
+  if (!sm->lex[level]) return planar_to_host(sm, level, host_out);
+  B200_SMEAR_CHECK(cudaMemcpyAsync(host_out, sm->lex[level], nreal_cfg(sm) * sizeof(double), cudaMemcpyDeviceToHost, st));
   B200_SMEAR_CHECK(cudaStreamSynchronize(st));
   return 0;
 }

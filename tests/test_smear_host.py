@@ -48,3 +48,28 @@ def test_level_copy_is_made_on_the_plans_device(tmp_path):
     fake.cudaGetDevice(ctypes.byref(d))
     assert d.value == 1
     """)
+
+
+def test_host_copy_of_a_level_keeps_no_device_memory(tmp_path):
+    """get_config of a level leaves the device memory in use as it was, also
+    where there is none left for a copy in between, and puts the planar level in
+    the lexical order."""
+    run(tmp_path, """
+    sm = b200dwf.StoutSmear([4, 4, 4, 4], 0.1, 2)
+    u, p = array(nlink)
+    b200dwf.check(lib.b200_smear_set_config(sm.handle, p, 0, None))
+    used = fake.fake_used()
+    for level in range(3):
+        sm.config(level)
+    assert fake.fake_used() == used
+    fake.fake_limit(used)
+    fake.fake_count()
+    for level in range(2):
+        got = sm.config(level)
+        # entry k of link (mu, site) is double2 (9 mu + k) vol + site of its level
+        mu, site, k, c = np.ix_(range(4), range(256), range(9), range(2))
+        want = 2 * ((9 * mu + k) * 256 + site) + c
+        got = got.reshape(4, 256, 9, 2)
+        assert np.array_equal(got - got[0, 0, 0, 0], want), level
+    assert fake.fake_used() == used
+    """)
