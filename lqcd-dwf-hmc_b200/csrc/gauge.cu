@@ -403,7 +403,7 @@ cudaError_t device_malloc_bytes(void** p, size_t n) {
   if (e != cudaErrorMemoryAllocation) return e;
   gauge_scratch_trim();
   const cudaError_t e2 = cudaMalloc(p, n);
-  if (e2 == cudaSuccess) cudaGetLastError();    // the first failure is over
+  cudaGetLastError();      // the caller reports it; left set, the next launch would too
   return e2;
 }
 

@@ -62,4 +62,5 @@ force()                                         # no room for scratch: still run
 fake.fake_limit(0)
 for k in range(3):                              # really out of memory: an error
     assert lib.b200_dwf_create(ctypes.byref(ctypes.c_void_p()), lat, 8, 0.1, 1.8, None, None, 1.0, lat) == -3
+b200dwf.check(lib.b200_momentum_update(lat, 0.1, pf, pu, None))     # and not this call's
 """)
