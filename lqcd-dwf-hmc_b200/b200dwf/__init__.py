@@ -383,15 +383,15 @@ class ScratchUser:
     """Base of the objects whose calls use the scratch that the library keeps
     between gauge forces; the last of them to go gives it back."""
 
-    _users = 0
+    _users = [0]
 
     def __new__(cls, *args, **kw):
-        ScratchUser._users += 1
+        cls._users[0] += 1
         return super().__new__(cls)
 
     def __del__(self):
-        ScratchUser._users -= 1
-        if ScratchUser._users == 0 and _lib is not None:
+        self._users[0] -= 1
+        if self._users[0] == 0 and _lib is not None:
             _lib.b200_scratch_release()
 
 

@@ -394,6 +394,20 @@ void set_last_error(int code, const char* fmt, ...);
     }                                                                               \
   } while (0)
 
+// Queues work on a stream of its own and waits for it, so that what is in
+// progress on the caller's streams is not touched (the levels are complete when
+// set_config returns).
+template <class F>
+static cudaError_t on_own_stream(F queue) {
+  cudaStream_t st = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = queue(st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  return e != cudaSuccess ? e : es;
+}
+
 static size_t nreal_cfg(const b200_smear* sm) { return 18 * 4 * sm->g.vol; }
 
 extern "C" {
@@ -510,18 +524,10 @@ struct OnPlanDevice {
   }
 };
 
-// Planar level -> lexical `out`, on a stream of its own, so that work in
-// progress on the caller's streams is not touched (the levels are complete when
-// set_config returns).
-static cudaError_t level_to_lex(const b200_smear* sm, int level, double* out) {
-  cudaStream_t st = nullptr;
-  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e != cudaSuccess) return e;
+// planar level -> lexical `out`
+static cudaError_t level_to_lex(const b200_smear* sm, int level, double* out, cudaStream_t st) {
   planar_to_links_kernel<<<link_grid(sm), 128, 0, st>>>(out, planar_level(sm, level));
-  e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaStreamDestroy(st);
-  return e;
+  return cudaGetLastError();
 }
 
 static int smear_fail(cudaError_t e, const char* what) {
@@ -534,7 +540,7 @@ static int make_lex(b200_smear* sm, int level) {
   OnPlanDevice on(sm);
   double* buf = nullptr;
   cudaError_t e = device_malloc(&buf, nreal_cfg(sm) * sizeof(double));
-  if (e == cudaSuccess) e = level_to_lex(sm, level, buf);
+  if (e == cudaSuccess) e = on_own_stream([&](cudaStream_t st) { return level_to_lex(sm, level, buf, st); });
   if (e != cudaSuccess) {
     cudaFree(buf);
     return smear_fail(e, "smear_config");
@@ -559,16 +565,19 @@ static int planar_to_host(b200_smear* sm, int level, double* host_out) {
   double* lex = nullptr;
   cudaError_t e = device_malloc(&lex, bytes);
   if (e == cudaSuccess) {
-    e = level_to_lex(sm, level, lex);
-    if (e == cudaSuccess) e = cudaMemcpy(host_out, lex, bytes, cudaMemcpyDeviceToHost);
+    e = on_own_stream([&](cudaStream_t st) {
+      const cudaError_t ek = level_to_lex(sm, level, lex, st);
+      return ek != cudaSuccess ? ek : cudaMemcpyAsync(host_out, lex, bytes, cudaMemcpyDeviceToHost, st);
+    });
     cudaFree(lex);
     return e == cudaSuccess ? 0 : smear_fail(e, "smear_get_config");
   }
   if (e != cudaErrorMemoryAllocation) return smear_fail(e, "smear_get_config");
-  cudaGetLastError();
   double2* planar = new (std::nothrow) double2[36 * vol];
   if (!planar) return smear_fail(cudaErrorMemoryAllocation, "smear_get_config");
-  e = cudaMemcpy(planar, planar_level(sm, level).p, bytes, cudaMemcpyDeviceToHost);
+  e = on_own_stream([&](cudaStream_t st) {
+    return cudaMemcpyAsync(planar, planar_level(sm, level).p, bytes, cudaMemcpyDeviceToHost, st);
+  });
   if (e == cudaSuccess)
     for (size_t mu = 0; mu < 4; ++mu)
       for (size_t site = 0; site < vol; ++site)
